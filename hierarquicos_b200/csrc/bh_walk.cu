@@ -26,7 +26,9 @@
 //    at m*q/m, level-L leaves are summed particle by particle.  Used to check
 //    the tree against the reference and to count the reference's interactions.
 #include <math.h>
+#include <stdint.h>
 
+#include "bh_fp64.cuh"
 #include "bh_internal.cuh"
 
 namespace bh {
@@ -46,6 +48,7 @@ constexpr int kCellQ = 64;
 constexpr int kBodyPerLane = 16;
 constexpr int kBodyQ = 32 + kWarp * kBodyPerLane;  // 544
 constexpr unsigned kFull = 0xffffffffu;
+constexpr int32_t kNoChild = 0x7fffffff;  // unused entry of a node's child list (records_kernel)
 
 template <typename T> struct Ops;
 template <> struct Ops<float> {
@@ -69,11 +72,25 @@ __device__ __forceinline__ void kahan_add(T &s, T &c, T x) {
 
 template <int ORDER> struct StageWords { static constexpr int value = ORDER >= 8 ? 24 : (ORDER >= 4 ? 12 : 4); };
 
+template <typename T> struct __align__(16) Vec4 { T x, y, z, w; };
+
+// Shared memory of one tree walk: the queues, the members and the members'-MAC
+// candidates of the current group, and the top of the walk's stack.
+constexpr int kSamples = 8;         // members of the first look of the members' MAC
+constexpr int kStackWindow = 512;  // stack entries kept in shared memory (a power of two)
+template <typename T>
+struct __align__(16) WalkSmem {
+  Vec4<T> member[2 * kWarp];  // group-frame position of every target slot
+  Vec4<T> cand[kWarp];        // centre of mass and size^2 of the nodes to test
+  int window[kStackWindow];
+  int cellq[kCellQ];
+  int bodyq[kBodyQ];
+};
+
 template <typename T, int ORDER>
 struct __align__(16) WarpSmem {
   T stage[kWarp * StageWords<ORDER>::value];
-  int cellq[kCellQ];
-  int bodyq[kBodyQ];
+  WalkSmem<T> w;
 };
 
 struct WalkArgs {
@@ -102,6 +119,13 @@ struct WalkArgs {
   int g_begin, g_end;  // groups walked: [g_begin, g_end), g_end < 0 = all
   int pipeline;        // FP32: producer/consumer warp teams
 };
+
+// a predicated shared-memory store: no branch, whatever the lanes decide
+__device__ __forceinline__ void store_if(int *p, int v, bool yes) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q st.shared.s32 [%0], %1;\n\t}"
+               ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v), "r"((int)yes)
+               : "memory");
+}
 
 template <typename T>
 __device__ __forceinline__ T warp_min(T v) {
@@ -200,13 +224,26 @@ __device__ __forceinline__ void load_words(const double *p, double (&w)[W]) {
 
 // Reciprocal square root.  FP32: one approximate hardware instruction
 // (rel. error ~2^-22.9) with subnormals flushed: every input is a squared
-// distance in units of the root cube side, never subnormal.  FP64: rsqrt().
+// distance in units of the root cube side, never subnormal.  FP64: the
+// binomial series of bh_fp64.cuh (the same range holds; kEps2Max bounds it
+// above).
 __device__ __forceinline__ float fast_rsqrt(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ double fast_rsqrt(double x) { return rsqrt(x); }
+__device__ __forceinline__ double fast_rsqrt(double x) { return inv_sqrt64(x); }
+
+// m r^-3 from r^2
+__device__ __forceinline__ float mass_r3(float r2, float m) {
+  const float ri = fast_rsqrt(r2);
+  return (m * ri) * (ri * ri);
+}
+__device__ __forceinline__ double mass_r3(double r2, double m) { return mass_over_r3(r2, m); }
+
+// A softening beyond this (squared, in root sides) gives zero forces either
+// way; larger squares would leave the series' range.
+constexpr double kEps2Max = 1e250;
 
 // (2^-level)^2 = 2^(-2 level), exact, from the exponent bits (level <= 21)
 template <typename T> __device__ __forceinline__ T pow2_neg2(int level);
@@ -231,8 +268,7 @@ __device__ __forceinline__ void body_force(T sx, T sy, T sz, T sm, T rx, T ry, T
   const T dx = sx - rx, dy = sy - ry, dz = sz - rz;
   T r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
   if (!SOFT) r2 = max(r2, r2_floor<T>());
-  const T ri = fast_rsqrt(r2);
-  const T f = (sm * ri) * (ri * ri);
+  const T f = mass_r3(r2, sm);
   bx = fma(f, dx, bx); by = fma(f, dy, by); bz = fma(f, dz, bz);
 }
 
@@ -390,43 +426,77 @@ struct WalkCounters {
 // queued as cells and the bodies of opened leaves and lone particles as
 // bodies; eval_cells(end, k) / eval_bodies(end, k) consume the k queue entries
 // that end at position `end`, 32 at a time and the remainders at the end.
-// Positions are relative to the group centre gc in units of the root side.
-// An accepted node of at most ASB bodies is queued as its bodies: for the
-// octupole, whose cell term costs as much as about 8 body terms, that is
-// cheaper and exact.
-template <typename T, int TPL, int ASB, typename CellsFn, typename BodiesFn>
-__device__ __forceinline__ void tree_walk(const WalkArgs &a, int *cellq, int *bodyq,
-                                          int32_t *stack, int stack_cap, int gf, int gn, int root,
+// Positions are relative to the group centre gc in units of the root side;
+// S.member holds the group's targets (32 TPL slots, unused ones repeating the
+// first target).  An accepted node of at most ASB bodies is queued as its
+// bodies: for the octupole, whose cell term costs as much as about 8 body
+// terms, that is cheaper and exact.
+//
+// Bound: latency; one pass over 32 nodes is a chain of dependent steps.  The
+// members' MAC candidates share the warp (one at a time they took 4,000 of the
+// 10,200 cycles of a pass at N = 1,024, where 14 of the 32 nodes are
+// candidates; now 860), the stack's top kStackWindow entries stay in shared
+// memory (older ones move to the global stack), one scan places both the
+// children and the bodies of a pass, and the appends are predicated stores.
+// EAGER walks (few groups, nothing else to hide the latency behind) load the
+// next pass's records, every node's children among them, before handing this
+// pass's batches on, and refuse most candidates by a look at kSamples members:
+// about 3,500 cycles a pass.  With many groups the extra loads and tests only
+// take issue slots from the consumers (2^20 bodies: 5.17 ms without, 5.29 with).
+template <typename T, int TPL, int ASB, bool EAGER, typename CellsFn, typename BodiesFn>
+__device__ __forceinline__ void tree_walk(const WalkArgs &a, WalkSmem<T> &S, int32_t *stack,
+                                          int stack_cap, int gf, int gn, int root,
                                           const double gc[3], double inv_s, const T blo[3],
                                           const T bhi[3], T theta2, T inv_theta2, T diag, T rad,
-                                          const T (&rx)[TPL], const T (&ry)[TPL],
-                                          const T (&rz)[TPL], WalkCounters &wc,
-                                          CellsFn &&eval_cells, BodiesFn &&eval_bodies) {
+                                          WalkCounters &wc, CellsFn &&eval_cells,
+                                          BodiesFn &&eval_bodies) {
   const int lane = threadIdx.x & (kWarp - 1);
   const unsigned lt = (1u << lane) - 1u;
-  int top = 1, ncell = 0, nbody = 0;
+  // distance at which a node of level `lane` passes the MAC
+  const T reach_of_level = sqrt(pow2_neg2<T>(min(lane, kMaxDepth)) * inv_theta2);
+  // stack entries [low, top) are in the window, [0, low) in global memory
+  int top = 1, low = 0, ncell = 0, nbody = 0;
   // a tree visits every node at most once per group: more tests than nodes
   // means a malformed tree, and the walk stops with an error instead of
   // looping
-  const int64_t max_tests = (int64_t)a.sc->n_compact + kWarp;
-  int64_t group_tests = 0;
+  const int max_tests = a.sc->n_compact + kWarp;
+  int group_tests = 0;
   if (root < 0) top = 0;  // a lone body: no tree, no force
-  if (lane == 0) stack[0] = root;
+  if (lane == 0) S.window[0] = root;
   __syncwarp();
-  while (top > 0) {
-    if (group_tests > max_tests) { wc.err |= kErrIndex; break; }
-    const int take = min(top, kWarp);
+  // the nodes of the next pass (the top of the stack) and their records
+  int take = 0, node = -1;
+  int4 mt = make_int4(0, 0, 0, 0), c0 = mt, c1 = mt;
+  double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+  auto fetch = [&]() {
+    take = min(top, kWarp);
     const int base = top - take;
-    const int node = lane < take ? stack[base + lane] : -1;
+    if (base < low) {  // older entries come back from the global stack
+      const int from = max(0, low - kStackWindow / 2);
+      for (int i = from + lane; i < low; i += kWarp) S.window[i & (kStackWindow - 1)] = stack[i];
+      low = from;
+      __syncwarp();
+    }
+    node = lane < take ? S.window[(base + lane) & (kStackWindow - 1)] : -1;
     top = base;
-    __syncwarp();
-    int cls = 0;  // 1 cell, 2 open leaf, 3 open internal
-    int4 mt = make_int4(0, 0, 0, 0);
-    T dx = (T)0, dy = (T)0, dz = (T)0, size2 = (T)0;
-    bool cand = false;
     if (node >= 0) {
       mt = a.meta[node];
-      const double4 c = a.com[node];
+      c = a.com[node];
+      if (EAGER) {
+        const int4 *cp = reinterpret_cast<const int4 *>(a.child + 8 * (int64_t)node);
+        c0 = cp[0]; c1 = cp[1];
+      }
+    }
+    __syncwarp();
+  };
+  fetch();
+  while (take > 0) {
+    if (group_tests > max_tests) { wc.err |= kErrIndex; break; }
+    int cls = 0;  // 1 cell, 2 open leaf, 3 open internal
+    T dx = (T)0, dy = (T)0, dz = (T)0, size2 = (T)0;
+    bool cand = false;
+    const T reach = __shfl_sync(kFull, reach_of_level, mt.z);
+    if (node >= 0) {
       dx = (T)((c.x - gc[0]) * inv_s); dy = (T)((c.y - gc[1]) * inv_s); dz = (T)((c.z - gc[2]) * inv_s);
       const T ex = max(max(blo[0] - dx, (T)0), dx - bhi[0]);
       const T ey = max(max(blo[1] - dy, (T)0), dy - bhi[1]);
@@ -442,7 +512,6 @@ __device__ __forceinline__ void tree_walk(const WalkArgs &a, int *cellq, int *bo
           // Every member is at least |c| - rad from the centre of mass (the
           // sphere bound); otherwise the members are tested one by one below
           // if the nearest of them (at most `diag` beyond the box) may pass.
-          const T reach = sqrt(size2 * inv_theta2);
           const T dc = sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
           if (dc - rad >= reach) {
             cls = 1;
@@ -454,109 +523,327 @@ __device__ __forceinline__ void tree_walk(const WalkArgs &a, int *cellq, int *bo
       }
     }
     // members' own MAC (morton_octree.f90:701-706: size^2 <= theta^2 d^2 with
-    // d from the member to the centre of mass), all members at once
-    for (unsigned pend = __ballot_sync(kFull, cand); pend; pend &= pend - 1) {
-      const int src = __ffs(pend) - 1;
-      const T cx = __shfl_sync(kFull, dx, src), cy = __shfl_sync(kFull, dy, src),
-              cz = __shfl_sync(kFull, dz, src), cs2 = __shfl_sync(kFull, size2, src);
+    // d from the member to the centre of mass).  Every lane first tests its own
+    // node against a few members spread over the group, which refuses most;
+    // the remaining candidates are gathered and share the warp: 2^sh lanes per
+    // candidate, each over its part of the members (interleaved, so that the
+    // reads of one step are adjacent), four at a time.
+    if (EAGER && __any_sync(kFull, cand)) {
       T dmin = (T)INFINITY;
 #pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        const T ux = cx - rx[t], uy = cy - ry[t], uz = cz - rz[t];
+      for (int k = 0; k < kSamples; ++k) {
+        const Vec4<T> q = S.member[k * (kWarp * TPL / kSamples)];
+        const T ux = dx - q.x, uy = dy - q.y, uz = dz - q.z;
         dmin = min(dmin, fma(ux, ux, fma(uy, uy, uz * uz)));
       }
-      dmin = warp_min(dmin);
-      if (lane == src && cs2 <= theta2 * dmin) cls = 1;
+      cand = cand && size2 <= theta2 * dmin;
+    }
+    const unsigned pend = __ballot_sync(kFull, cand);
+    if (pend) {
+      const int nc = __popc(pend), rank = __popc(pend & lt);
+      if (cand) S.cand[rank] = Vec4<T>{dx, dy, dz, size2};
+      __syncwarp();
+      const int sh = min(__clz(nc - 1) - 27, TPL == 2 ? 4 : 3);  // 5 - ceil(log2 nc)
+      const int step = 1 << sh;
+      const Vec4<T> t = S.cand[min(lane >> sh, nc - 1)];
+      T dm[4] = {(T)INFINITY, (T)INFINITY, (T)INFINITY, (T)INFINITY};
+      for (int i = lane & (step - 1); i < kWarp * TPL; i += 4 * step) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const Vec4<T> q = S.member[i + k * step];
+          const T ux = t.x - q.x, uy = t.y - q.y, uz = t.z - q.z;
+          dm[k] = min(dm[k], fma(ux, ux, fma(uy, uy, uz * uz)));
+        }
+      }
+      T dmin = min(min(dm[0], dm[1]), min(dm[2], dm[3]));
+      for (int o = step >> 1; o > 0; o >>= 1) dmin = min(dmin, __shfl_xor_sync(kFull, dmin, o));
+      const unsigned pass = __ballot_sync(kFull, t.w <= theta2 * dmin);
+      if (cand && ((pass >> (rank << sh)) & 1u)) cls = 1;
     }
     if (cls == 1 && mt.y <= ASB) cls = 2;
-    wc.tests += take;
     group_tests += take;
     // cells
     const unsigned cm = __ballot_sync(kFull, cls == 1);
-    if (cls == 1) cellq[ncell + __popc(cm & lt)] = node;
+    store_if(&S.cellq[ncell + __popc(cm & lt)], node, cls == 1);
     ncell += __popc(cm);
-    // children of opened internal nodes
-    int32_t ch[8];
-    int nnc = 0, npc = 0;
-    if (cls == 3) {
+    // children of opened internal nodes; bodies: lone-particle children (<= 8)
+    // and leaf ranges, kBodyPerLane at a time.  A child entry is a node (>= 0),
+    // a particle (< 0) or unused (kNoChild).
+    if (!EAGER && cls == 3) {
       const int4 *cp = reinterpret_cast<const int4 *>(a.child + 8 * (int64_t)node);
-      const int4 c0 = cp[0], c1 = cp[1];
-      ch[0] = c0.x; ch[1] = c0.y; ch[2] = c0.z; ch[3] = c0.w;
-      ch[4] = c1.x; ch[5] = c1.y; ch[6] = c1.z; ch[7] = c1.w;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (c < mt.w) { if (ch[c] >= 0) ++nnc; else ++npc; }
+      c0 = cp[0]; c1 = cp[1];
     }
-    int tot;
-    const int soff = warp_excl_scan(nnc, lane, tot);
+    const int32_t ch[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    const bool open = cls == 3;
+    int nnc = 0, npc = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      nnc += (unsigned)ch[k] < (unsigned)kNoChild ? 1 : 0;
+      npc += ch[k] < 0 ? 1 : 0;
+    }
+    int rf = mt.x, rn = cls == 2 ? mt.y : 0;
+    int give = open ? npc : min(rn, kBodyPerLane);
+    int both;
+    const int off = warp_excl_scan((open ? nnc : 0) | (give << 16), lane, both);
+    const int tot = both & 0xffff;
+    int btot = both >> 16;
+    int boff = nbody + (off >> 16);
     if (top + tot > stack_cap) {
       // capacity exceeded: the group's result is incomplete and flagged;
       // the host repeats the walk with a larger stack
       wc.err |= kErrStackOverflow;
     } else {
-      if (cls == 3) {
-        int k = top + soff;
+      if (top + tot - low > kStackWindow) {  // the oldest entries move out
+        const int to = max(low, top - kStackWindow / 4);
+        for (int i = low + lane; i < to; i += kWarp) stack[i] = S.window[i & (kStackWindow - 1)];
+        low = to;
+        __syncwarp();
+      }
+      if (tot > 0) {
+        int k = top + (off & 0xffff);
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < mt.w && ch[c] >= 0) stack[k++] = ch[c];
+        for (int q = 0; q < 8; ++q) {
+          const bool is = open && (unsigned)ch[q] < (unsigned)kNoChild;
+          store_if(&S.window[k & (kStackWindow - 1)], ch[q], is);
+          k += is ? 1 : 0;
+        }
       }
       top += tot;
     }
-    // bodies: lone-particle children (<= 8, one pass) and leaf ranges
-    int rf = 0, rn = 0;
-    if (cls == 2) { rf = mt.x; rn = mt.y; }
-    bool first_pass = true;
-    // nothing to queue on any lane (the common case): no scan
-    for (bool any = __ballot_sync(kFull, rn > 0 || (cls == 3 && npc > 0)) != 0u; any;
-         any = __ballot_sync(kFull, rn > 0) != 0u) {
-      int give;
-      if (first_pass && cls == 3) give = npc;
-      else give = min(rn, kBodyPerLane);
-      int btot;
-      const int boff = warp_excl_scan(give, lane, btot);
-      if (btot == 0) break;
-      if (first_pass && cls == 3) {
-        int k = nbody + boff;
+    if (btot > 0) {
+      int k = boff;
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < mt.w && ch[c] < 0) bodyq[k++] = ~ch[c];
-      } else {
-        for (int k = 0; k < give; ++k) bodyq[nbody + boff + k] = rf + k;
-        rf += give; rn -= give;
+      for (int q = 0; q < 8; ++q) {
+        const bool is = open && ch[q] < 0;
+        store_if(&S.bodyq[k], ~ch[q], is);
+        k += is ? 1 : 0;
       }
-      first_pass = false;
-      nbody += btot;
-      __syncwarp();
-      while (nbody >= kWarp) { eval_bodies(nbody, kWarp); nbody -= kWarp; }
     }
     __syncwarp();
+    // the next pass's records load while this one's batches are handed on
+    if (EAGER) fetch();
+    if (btot > 0) {
+      if (open) give = 0;
+      for (;;) {
+#pragma unroll
+        for (int k = 0; k < kBodyPerLane / 2; ++k) store_if(&S.bodyq[boff + k], rf + k, k < give);
+        if (__any_sync(kFull, give > kBodyPerLane / 2)) {
+#pragma unroll
+          for (int k = kBodyPerLane / 2; k < kBodyPerLane; ++k)
+            store_if(&S.bodyq[boff + k], rf + k, k < give);
+        }
+        rf += give; rn -= give;
+        nbody += btot;
+        __syncwarp();
+        while (nbody >= kWarp) { eval_bodies(nbody, kWarp); nbody -= kWarp; }
+        if (__ballot_sync(kFull, rn > 0) == 0u) break;
+        give = min(rn, kBodyPerLane);
+        boff = nbody + warp_excl_scan(give, lane, btot);
+      }
+    }
     while (ncell >= kWarp) { eval_cells(ncell, kWarp); ncell -= kWarp; }
     __syncwarp();
+    if (!EAGER) fetch();
   }
+  wc.tests += group_tests;
   if (ncell > 0) eval_cells(ncell, ncell);
   if (nbody > 0) eval_bodies(nbody, nbody);
 }
 
-// One group: TPL targets per lane (the group has <= 32 * TPL bodies).
-template <typename T, int ORDER, int TPL, bool SOFT>
-__device__ __forceinline__ void walk_group(const WalkArgs &a, WarpSmem<T, ORDER> &S,
-                                           int32_t *stack, int stack_cap, int gf, int gn,
-                                           const SysScalars &ss, T theta2, WalkCounters &wc) {
-  const double inv_s = 1.0 / ss.ssa, inv_m = 1.0 / ss.mass;
-  const double nq = inv_m * inv_s * inv_s, no = nq * inv_s;
-  const T eps2 = (T)(a.eps2 * inv_s * inv_s);
-  const int root = ss.root;
-  constexpr int W = StageWords<ORDER>::value;
-  constexpr bool kKahan = sizeof(T) == 4;
-  const int lane = threadIdx.x & (kWarp - 1);
+// A lane's TPL targets in the group frame, as the evaluation reads them: the
+// FP32 walk wants them negated in both halves of a pair.
+template <typename T, int TPL> struct Targets {
+  T x[TPL], y[TPL], z[TPL];
+  __device__ __forceinline__ void set(int t, T a, T b, T c) { x[t] = a; y[t] = b; z[t] = c; }
+};
+template <int TPL> struct Targets<float, TPL> {
+  float2 x[TPL], y[TPL], z[TPL];
+  __device__ __forceinline__ void set(int t, float a, float b, float c) {
+    x[t] = splat(-a); y[t] = splat(-b); z[t] = splat(-c);
+  }
+};
 
+// Staging of one batch, lane j entry j (j < n).  FP64: entry j at [W j, W (j + 1)).
+// FP32: entries 2i and 2i + 1 interleaved word by word at [2W i, 2W (i + 1)), an odd
+// count padded with an empty far entry.
+template <typename T, int ORDER>
+__device__ __forceinline__ void stage_cells(T *stage, int lane, int nc, int node, const WalkArgs &a,
+                                            const double gc[3], double inv_s, double inv_m,
+                                            double nq, double no) {
+  constexpr int W = StageWords<ORDER>::value;
+  if constexpr (sizeof(T) == 4) {
+    float *w = stage + (lane >> 1) * 2 * W + (lane & 1);
+    if (lane < nc) {
+      stage_cell<float, ORDER, 2>(w, node, a, gc, inv_s, inv_m, nq, no);
+    } else if (lane == nc && (nc & 1)) {
+#pragma unroll
+      for (int k = 3; k < W; ++k) w[2 * k] = 0.0f;
+      w[0] = w[2] = w[4] = kPadPos;
+    }
+  } else {
+    if (lane < nc) stage_cell<T, ORDER>(stage + lane * W, node, a, gc, inv_s, inv_m, nq, no);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void stage_bodies(T *stage, int lane, int nb, int body, const WalkArgs &a,
+                                             const double gc[3], double inv_s, double inv_m) {
+  constexpr int STR = sizeof(T) == 4 ? 2 : 1;
+  T *w = sizeof(T) == 4 ? stage + (lane >> 1) * 8 + (lane & 1) : stage + lane * 4;
+  if (lane < nb) {
+    const double4 s = a.spos[body];
+    w[0] = (T)((s.x - gc[0]) * inv_s);
+    w[STR] = (T)((s.y - gc[1]) * inv_s);
+    w[2 * STR] = (T)((s.z - gc[2]) * inv_s);
+    w[3 * STR] = (T)(s.w * inv_m);
+  } else if (sizeof(T) == 4 && lane == nb && (nb & 1)) {
+    w[0] = w[STR] = w[2 * STR] = (T)kPadPos;
+    w[3 * STR] = (T)0;
+  }
+}
+
+// The sum of one staged batch for every target of the lane.
+template <typename T, int ORDER, int TPL>
+__device__ __forceinline__ void sum_cells(const T *stage, int nc, const Targets<T, TPL> &g, T eps2,
+                                          T (&sx)[TPL], T (&sy)[TPL], T (&sz)[TPL]) {
+  constexpr int W = StageWords<ORDER>::value;
+  if constexpr (sizeof(T) == 4) {
+    const float2 eps2p = splat(eps2);
+    float2 bx[TPL], by[TPL], bz[TPL];
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
+    const int np = (nc + 1) >> 1;
+#pragma unroll 2
+    for (int j = 0; j < np; ++j) {
+      const float4 *st = reinterpret_cast<const float4 *>(stage) + j * (W / 2);
+      float2 cw[W];
+#pragma unroll
+      for (int k = 0; k < W / 2; ++k) {
+        const float4 v = st[k];
+        cw[2 * k] = make_float2(v.x, v.y);
+        cw[2 * k + 1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int t = 0; t < TPL; ++t)
+        cell_force2<ORDER>(cw, g.x[t], g.y[t], g.z[t], eps2p, bx[t], by[t], bz[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      sx[t] = bx[t].x + bx[t].y; sy[t] = by[t].x + by[t].y; sz[t] = bz[t].x + bz[t].y;
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) sx[t] = sy[t] = sz[t] = (T)0;
+#pragma unroll 2
+    for (int j = 0; j < nc; ++j) {
+      T w[W];
+      load_words<W>(stage + j * W, w);
+#pragma unroll
+      for (int t = 0; t < TPL; ++t)
+        cell_force<T, ORDER>(w, g.x[t], g.y[t], g.z[t], eps2, sx[t], sy[t], sz[t]);
+    }
+  }
+}
+template <typename T, int TPL, bool SOFT>
+__device__ __forceinline__ void sum_bodies(const T *stage, int nb, const Targets<T, TPL> &g, T eps2,
+                                           T (&sx)[TPL], T (&sy)[TPL], T (&sz)[TPL]) {
+  if constexpr (sizeof(T) == 4) {
+    const float2 eps2p = splat(eps2);
+    float2 bx[TPL], by[TPL], bz[TPL];
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
+    const int np = (nb + 1) >> 1;
+    const float4 *st = reinterpret_cast<const float4 *>(stage);
+    for (int j = 0; j < np; ++j) {
+      const float4 u = st[2 * j], v = st[2 * j + 1];
+      const float2 px = make_float2(u.x, u.y), py = make_float2(u.z, u.w);
+      const float2 pz = make_float2(v.x, v.y), pm = make_float2(v.z, v.w);
+#pragma unroll
+      for (int t = 0; t < TPL; ++t)
+        body_force2<SOFT>(px, py, pz, pm, g.x[t], g.y[t], g.z[t], eps2p, bx[t], by[t], bz[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      sx[t] = bx[t].x + bx[t].y; sy[t] = by[t].x + by[t].y; sz[t] = bz[t].x + bz[t].y;
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) sx[t] = sy[t] = sz[t] = (T)0;
+#pragma unroll 2
+    for (int j = 0; j < nb; ++j) {
+      T w[4];
+      load_words<4>(stage + j * 4, w);
+#pragma unroll
+      for (int t = 0; t < TPL; ++t)
+        body_force<T, SOFT>(w[0], w[1], w[2], w[3], g.x[t], g.y[t], g.z[t], eps2, sx[t], sy[t], sz[t]);
+    }
+  }
+}
+
+// Running sums of a lane's targets: Kahan-compensated in FP32.
+template <typename T, int TPL> struct Sums {
+  static constexpr bool kKahan = sizeof(T) == 4;
+  T ax[TPL], ay[TPL], az[TPL], cx[TPL], cy[TPL], cz[TPL];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) ax[t] = ay[t] = az[t] = cx[t] = cy[t] = cz[t] = (T)0;
+  }
+  __device__ __forceinline__ void add(const T (&sx)[TPL], const T (&sy)[TPL], const T (&sz)[TPL]) {
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      if (kKahan) {
+        kahan_add(ax[t], cx[t], sx[t]); kahan_add(ay[t], cy[t], sy[t]); kahan_add(az[t], cz[t], sz[t]);
+      } else {
+        ax[t] += sx[t]; ay[t] += sy[t]; az[t] += sz[t];
+      }
+    }
+  }
+  // forces in the original order; every system's result is an (n_s, 3)
+  // Fortran-ordered block at 3 * off_s
+  __device__ __forceinline__ void write(const WalkArgs &a, const SysScalars &ss, int gf, int gn,
+                                        int lane) const {
+    const double inv_s = 1.0 / ss.ssa;
+    const double scale = a.G * ss.mass * inv_s * inv_s;
+    double *out = a.out + 3 * ss.off;
+    const int64_t ns = ss.n;
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      if (lane + kWarp * t >= gn) continue;
+      const int i = gf + lane + kWarp * t;
+      const int64_t p = a.perm[i] - ss.off;
+      double fxs = (double)ax[t], fys = (double)ay[t], fzs = (double)az[t];
+      if (kKahan) { fxs -= (double)cx[t]; fys -= (double)cy[t]; fzs -= (double)cz[t]; }
+      double sc = scale;
+      if (a.out_kind == 0) sc *= a.spos[i].w;
+      out[p] = fxs * sc;
+      out[ns + p] = fys * sc;
+      out[2 * ns + p] = fzs * sc;
+    }
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ T group_eps2(const WalkArgs &a, double inv_s) {
+  const double e2 = a.eps2 * inv_s * inv_s;
+  return (T)(sizeof(T) == 8 ? fmin(e2, kEps2Max) : e2);
+}
+
+// The frame of one group (its <= 32 TPL bodies start at gf): centre gc and box
+// of the members, which go to S.member, and the tree walk with the given
+// consumers of the queues.
+template <typename T, int ORDER, int TPL, bool EAGER, typename CellsFn, typename BodiesFn,
+          typename BeginFn>
+__device__ __forceinline__ void walk_members(const WalkArgs &a, WalkSmem<T> &S, int32_t *stack,
+                                             int stack_cap, int gf, int gn, const SysScalars &ss,
+                                             T theta2, double gc[3], WalkCounters &wc,
+                                             BeginFn &&begin, CellsFn &&eval_cells,
+                                             BodiesFn &&eval_bodies) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const double inv_s = 1.0 / ss.ssa;
   double px[TPL], py[TPL], pz[TPL];
-  bool valid[TPL];
 #pragma unroll
   for (int t = 0; t < TPL; ++t) {
     const int k = lane + kWarp * t;
-    valid[t] = k < gn;
-    const double4 p = a.spos[gf + (valid[t] ? k : 0)];
+    const double4 p = a.spos[gf + (k < gn ? k : 0)];
     px[t] = p.x; py[t] = p.y; pz[t] = p.z;
   }
   double lo[3] = {px[0], py[0], pz[0]}, hi[3] = {px[0], py[0], pz[0]};
@@ -566,18 +853,15 @@ __device__ __forceinline__ void walk_group(const WalkArgs &a, WarpSmem<T, ORDER>
     lo[1] = fmin(lo[1], py[t]); hi[1] = fmax(hi[1], py[t]);
     lo[2] = fmin(lo[2], pz[t]); hi[2] = fmax(hi[2], pz[t]);
   }
-  double gc[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) gc[k] = 0.5 * (warp_min(lo[k]) + warp_max(hi[k]));
-  T rx[TPL], ry[TPL], rz[TPL];
-  T ax[TPL], ay[TPL], az[TPL], cx[TPL], cy[TPL], cz[TPL];
-  T blo[3], bhi[3];
+  T rx[TPL], ry[TPL], rz[TPL], blo[3], bhi[3];
 #pragma unroll
   for (int t = 0; t < TPL; ++t) {
     rx[t] = (T)((px[t] - gc[0]) * inv_s);
     ry[t] = (T)((py[t] - gc[1]) * inv_s);
     rz[t] = (T)((pz[t] - gc[2]) * inv_s);
-    ax[t] = ay[t] = az[t] = cx[t] = cy[t] = cz[t] = (T)0;
+    S.member[lane + kWarp * t] = Vec4<T>{rx[t], ry[t], rz[t], (T)0};
     if (t == 0) { blo[0] = bhi[0] = rx[0]; blo[1] = bhi[1] = ry[0]; blo[2] = bhi[2] = rz[0]; }
     else {
       blo[0] = min(blo[0], rx[t]); bhi[0] = max(bhi[0], rx[t]);
@@ -596,167 +880,52 @@ __device__ __forceinline__ void walk_group(const WalkArgs &a, WarpSmem<T, ORDER>
 #pragma unroll
   for (int t = 0; t < TPL; ++t) rad2 = max(rad2, fma(rx[t], rx[t], fma(ry[t], ry[t], rz[t] * rz[t])));
   const T rad = sqrt(warp_max(rad2));
+  begin(rx, ry, rz);
+  tree_walk<T, TPL, bodies_as_cell<ORDER>(), EAGER>(a, S, stack, stack_cap, gf, gn, ss.root, gc, inv_s,
+                                             blo, bhi, theta2, inv_theta2, diag, rad, wc,
+                                             eval_cells, eval_bodies);
+}
 
-  auto accumulate = [&](const T (&bx)[TPL], const T (&by)[TPL], const T (&bz)[TPL]) {
+// One group on one warp: TPL targets per lane.
+template <typename T, int ORDER, int TPL, bool SOFT>
+__device__ __forceinline__ void walk_group(const WalkArgs &a, WarpSmem<T, ORDER> &S,
+                                           int32_t *stack, int stack_cap, int gf, int gn,
+                                           const SysScalars &ss, T theta2, WalkCounters &wc) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const double inv_s = 1.0 / ss.ssa, inv_m = 1.0 / ss.mass;
+  const double nq = inv_m * inv_s * inv_s, no = nq * inv_s;
+  const T eps2 = group_eps2<T>(a, inv_s);
+  double gc[3];
+  Targets<T, TPL> tg;
+  Sums<T, TPL> acc;
+  acc.clear();
+  walk_members<T, ORDER, TPL, false>(
+      a, S.w, stack, stack_cap, gf, gn, ss, theta2, gc, wc,
+      [&](const T (&rx)[TPL], const T (&ry)[TPL], const T (&rz)[TPL]) {
 #pragma unroll
-    for (int t = 0; t < TPL; ++t) {
-      if (kKahan) {
-        kahan_add(ax[t], cx[t], bx[t]); kahan_add(ay[t], cy[t], by[t]); kahan_add(az[t], cz[t], bz[t]);
-      } else {
-        ax[t] += bx[t]; ay[t] += by[t]; az[t] += bz[t];
-      }
-    }
-  };
-  // FP32: paired evaluation; target coordinates negated and duplicated once
-  constexpr bool kPaired = sizeof(T) == 4;
-  float2 nrx[TPL], nry[TPL], nrz[TPL];
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    nrx[t] = splat(-(float)rx[t]); nry[t] = splat(-(float)ry[t]); nrz[t] = splat(-(float)rz[t]);
-  }
-  const float2 eps2p = splat((float)eps2);
-  // evaluate the nb queue entries ending at position `end`
-  auto eval_bodies = [&](int end, int nb) {
-    if constexpr (kPaired) {
-      // stage: body pair i at [8i, 8i + 8) as (x, x', y, y', z, z', m, m'); an
-      // odd count is padded with a massless far body
-      float *w = reinterpret_cast<float *>(S.stage) + (lane >> 1) * 8 + (lane & 1);
-      if (lane < nb) {
-        const int p = S.bodyq[end - nb + lane];
-        const double4 s = a.spos[p];
-        w[0] = (float)((s.x - gc[0]) * inv_s);
-        w[2] = (float)((s.y - gc[1]) * inv_s);
-        w[4] = (float)((s.z - gc[2]) * inv_s);
-        w[6] = (float)(s.w * inv_m);
-      } else if (lane == nb && (nb & 1)) {
-        w[0] = w[2] = w[4] = kPadPos;
-        w[6] = 0.0f;
-      }
-      __syncwarp();
-      float2 bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
-      const int np = (nb + 1) >> 1;
-      const float4 *st = reinterpret_cast<const float4 *>(S.stage);
-      for (int j = 0; j < np; ++j) {
-        const float4 u = st[2 * j], v = st[2 * j + 1];
-        const float2 sx = make_float2(u.x, u.y), sy = make_float2(u.z, u.w);
-        const float2 sz = make_float2(v.x, v.y), sm = make_float2(v.z, v.w);
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-          body_force2<SOFT>(sx, sy, sz, sm, nrx[t], nry[t], nrz[t], eps2p, bx[t], by[t], bz[t]);
-      }
-      T sx[TPL], sy[TPL], sz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        sx[t] = bx[t].x + bx[t].y; sy[t] = by[t].x + by[t].y; sz[t] = bz[t].x + bz[t].y;
-      }
-      accumulate(sx, sy, sz);
-    } else {
-      if (lane < nb) {
-        const int p = S.bodyq[end - nb + lane];
-        const double4 s = a.spos[p];
-        T *w = S.stage + lane * 4;
-        w[0] = (T)((s.x - gc[0]) * inv_s);
-        w[1] = (T)((s.y - gc[1]) * inv_s);
-        w[2] = (T)((s.z - gc[2]) * inv_s);
-        w[3] = (T)(s.w * inv_m);
-      }
-      __syncwarp();
-      T bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = (T)0;
-#pragma unroll 2
-      for (int j = 0; j < nb; ++j) {
-        T w[4];
-        load_words<4>(S.stage + j * 4, w);
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-          body_force<T, SOFT>(w[0], w[1], w[2], w[3], rx[t], ry[t], rz[t], eps2, bx[t], by[t], bz[t]);
-      }
-      accumulate(bx, by, bz);
-    }
-    wc.pp += (unsigned long long)nb * gn;
-    __syncwarp();
-  };
-  auto eval_cells = [&](int end, int nc) {
-    if constexpr (kPaired) {
-      // stage: cell pair i at [2Wi, 2W(i + 1)), word k of both cells at 2k, 2k + 1;
-      // an odd count is padded with an empty far cell
-      float *w = reinterpret_cast<float *>(S.stage) + (lane >> 1) * 2 * W + (lane & 1);
-      if (lane < nc) {
-        stage_cell<float, ORDER, 2>(w, S.cellq[end - nc + lane], a, gc, inv_s, inv_m, nq, no);
-      } else if (lane == nc && (nc & 1)) {
-#pragma unroll
-        for (int k = 3; k < W; ++k) w[2 * k] = 0.0f;
-        w[0] = w[2] = w[4] = kPadPos;
-      }
-      __syncwarp();
-      float2 bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
-      const int np = (nc + 1) >> 1;
-#pragma unroll 2
-      for (int j = 0; j < np; ++j) {
-        const float4 *st = reinterpret_cast<const float4 *>(S.stage) + j * (W / 2);
-        float2 cw[W];
-#pragma unroll
-        for (int k = 0; k < W / 2; ++k) {
-          const float4 v = st[k];
-          cw[2 * k] = make_float2(v.x, v.y);
-          cw[2 * k + 1] = make_float2(v.z, v.w);
-        }
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-          cell_force2<ORDER>(cw, nrx[t], nry[t], nrz[t], eps2p, bx[t], by[t], bz[t]);
-      }
-      T sx[TPL], sy[TPL], sz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        sx[t] = bx[t].x + bx[t].y; sy[t] = by[t].x + by[t].y; sz[t] = bz[t].x + bz[t].y;
-      }
-      accumulate(sx, sy, sz);
-    } else {
-      if (lane < nc)
-        stage_cell<T, ORDER>(S.stage + lane * W, S.cellq[end - nc + lane], a, gc, inv_s, inv_m, nq, no);
-      __syncwarp();
-      T bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = (T)0;
-#pragma unroll 2
-      for (int j = 0; j < nc; ++j) {
-        T w[W];
-        load_words<W>(S.stage + j * W, w);
-#pragma unroll
-        for (int t = 0; t < TPL; ++t) cell_force<T, ORDER>(w, rx[t], ry[t], rz[t], eps2, bx[t], by[t], bz[t]);
-      }
-      accumulate(bx, by, bz);
-    }
-    wc.pc += (unsigned long long)nc * gn;
-    __syncwarp();
-  };
-
-  tree_walk<T, TPL, bodies_as_cell<ORDER>()>(a, S.cellq, S.bodyq, stack, stack_cap, gf, gn, root, gc, inv_s, blo, bhi,
-                    theta2, inv_theta2, diag, rad, rx, ry, rz, wc, eval_cells, eval_bodies);
-
-  // forces in the original order; every system's result is an (n_s, 3)
-  // Fortran-ordered block at 3 * off_s
-  const double scale = a.G * ss.mass * inv_s * inv_s;
-  double *out = a.out + 3 * ss.off;
-  const int64_t ns = ss.n;
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    if (!valid[t]) continue;
-    const int i = gf + lane + kWarp * t;
-    const int64_t p = a.perm[i] - ss.off;
-    double fxs = (double)ax[t], fys = (double)ay[t], fzs = (double)az[t];
-    if (kKahan) { fxs -= (double)cx[t]; fys -= (double)cy[t]; fzs -= (double)cz[t]; }
-    double sc = scale;
-    if (a.out_kind == 0) sc *= a.spos[i].w;
-    out[p] = fxs * sc;
-    out[ns + p] = fys * sc;
-    out[2 * ns + p] = fzs * sc;
-  }
+        for (int t = 0; t < TPL; ++t) tg.set(t, rx[t], ry[t], rz[t]);
+      },
+      [&](int end, int nc) {
+        stage_cells<T, ORDER>(S.stage, lane, nc, lane < nc ? S.w.cellq[end - nc + lane] : 0, a, gc,
+                              inv_s, inv_m, nq, no);
+        __syncwarp();
+        T sx[TPL], sy[TPL], sz[TPL];
+        sum_cells<T, ORDER, TPL>(S.stage, nc, tg, eps2, sx, sy, sz);
+        acc.add(sx, sy, sz);
+        wc.pc += (unsigned long long)nc * gn;
+        __syncwarp();
+      },
+      [&](int end, int nb) {
+        stage_bodies<T>(S.stage, lane, nb, lane < nb ? S.w.bodyq[end - nb + lane] : 0, a, gc, inv_s,
+                        inv_m);
+        __syncwarp();
+        T sx[TPL], sy[TPL], sz[TPL];
+        sum_bodies<T, TPL, SOFT>(S.stage, nb, tg, eps2, sx, sy, sz);
+        acc.add(sx, sy, sz);
+        wc.pp += (unsigned long long)nb * gn;
+        __syncwarp();
+      });
+  acc.write(a, ss, gf, gn, lane);
 }
 
 // Persistent warps, one per block, take groups from a global cursor until
@@ -793,43 +962,49 @@ group_walk_kernel(WalkArgs a) {
   }
 }
 
-// ---- warp-specialised FP32 group walk (pipeline = 1) ----
+// ---- warp-specialised group walk (pipeline = 1) ----
 //
-// A block holds kTeams teams of one producer warp and one consumer warp.
-// The producer takes groups from the global cursor, walks the tree exactly as
-// the one-warp walk does and stages every batch of 32 cells or bodies into a
-// ring of kRing shared-memory slots; its consumer evaluates the batches and
-// writes the forces.  Every target sees the batches of the one-warp walk in
-// the same order with the same arithmetic, so the results are the same bit
-// for bit; the tree walk of one group overlaps the evaluation of another.
-// Producers (warpgroup 0) hand registers to the consumers (warpgroup 1) with
-// setmaxnreg, so that more teams fit on an SM.  Each slot has a "full"
-// mbarrier (32 arrivals: the producer's lanes) and an "empty" one (32
-// arrivals: the consumer's lanes).  Every wait is bounded: a wait that lasts
-// more than about 2 s, or sees the block's abort flag, gives up, sets the flag
-// and reports an error; every warp of the block then leaves its loop.
+// A block is one producer warp and CONS consumer warps.  The producer
+// takes groups from the global cursor, walks the tree exactly as the one-warp
+// walk does and hands every batch of 32 cells or bodies on as a list of ids in
+// a ring of shared-memory slots.  Batch i belongs to consumer
+// i mod CONS, which loads and stages the entries itself (so no load of
+// theirs delays the walk), sums the batch for the group's targets and then, in
+// batch order, adds its sums to the running (Kahan) sums that the consumers
+// hand on to each other through shared memory.  Every target sees the batches
+// of the one-warp walk in the same order with the same arithmetic, so the
+// results are the same bit for bit; the tree walk of one group overlaps the
+// evaluation of the previous one, and a group's batches overlap one another.
+// Each slot has a "full" mbarrier (the producer's arrival), an "empty" one (its
+// consumer's, once the ids are read) and a "turn" one (the arrival of the
+// consumer of the batch before it, once its sums are added).  Every wait is
+// bounded: a wait that lasts more than about 2 s, or sees the block's abort
+// flag, gives up, sets the flag and reports an error; every warp of the block
+// then leaves its loop.
+// 7 consumers a block: N = 1,024 81 -> 30 us, 4,096 196 -> 79 us, 16,384 371 ->
+// 157 us against one team (below) per group; the FP64 walk at 65,536 bodies
+// (3 consumers, 4 blocks per SM) 2.37 -> 1.16 ms against one warp per group
+// evaluating its own batches.  launch_group_walk has the sizes where each wins.
 
-constexpr int kTeams = 4;
-constexpr int kRing = 4;
 constexpr long long kWaitCycles = 4000000000LL;
 constexpr int kRingStart = 1, kRingCells = 2, kRingBodies = 3, kRingEnd = 4, kRingQuit = 5;
 
-template <int ORDER>
-struct __align__(16) RingSlot {
-  int kind, count, g, unused;
+struct __align__(16) WideSlot {
+  int kind, count, g, first;  // first: nothing of the group was added before
   double gc[3];
-  double unused2;
-  float stage[kWarp * StageWords<ORDER>::value];
+  double unused;
+  int id[kWarp];
 };
 
-template <int ORDER>
-struct __align__(16) PipeSmem {
-  unsigned long long full[kTeams][kRing];
-  unsigned long long empty[kTeams][kRing];
+template <typename T, int ORDER, int CONS>
+struct __align__(16) WideSmem {
+  static constexpr int kSlots = 2 * CONS;  // of the ring
+  unsigned long long full[kSlots], empty[kSlots], turn[kSlots];
   int abort_flag;
-  int cellq[kTeams][kCellQ];
-  int bodyq[kTeams][kBodyQ];
-  RingSlot<ORDER> ring[kTeams][kRing];
+  WalkSmem<T> walk;
+  WideSlot ring[kSlots];
+  T sums[6][2 * kWarp];  // running sums of the group whose turn it is
+  T stage[CONS][kWarp * StageWords<ORDER>::value];
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
@@ -858,10 +1033,10 @@ __device__ __forceinline__ bool mbar_test(unsigned long long *b, unsigned parity
 __device__ __forceinline__ bool mbar_wait_warp(unsigned long long *b, unsigned parity,
                                                volatile int *abort_flag,
                                                long long limit = kWaitCycles) {
+  if (__all_sync(kFull, mbar_test(b, parity))) return true;
   const long long t0 = clock64();
   for (;;) {
-    const bool ok = mbar_test(b, parity);
-    if (__all_sync(kFull, ok)) return true;
+    if (__all_sync(kFull, mbar_test(b, parity))) return true;
     int stop = 0;
     if ((threadIdx.x & (kWarp - 1)) == 0) {
       if (*abort_flag) stop = 1;
@@ -871,266 +1046,387 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned long long *b, unsigned p
   }
 }
 
-// Producer side of one group: the target set-up and tree walk of walk_group,
-// with every batch staged into the ring.  `alive` turns false (for the rest
-// of the kernel) when a wait gave up.
-template <int ORDER, int TPL, bool SOFT>
-__device__ __forceinline__ void produce_group(const WalkArgs &a, PipeSmem<ORDER> &P, int team,
-                                              int &it, bool &alive, volatile int *abort_flag,
+// Producer side of one group: the walk of walk_group, with every batch's ids
+// put into the ring.  `alive` turns false (for the rest of the kernel) when a
+// wait gave up.
+template <typename T, int ORDER, int TPL, int CONS>
+__device__ __forceinline__ void wide_produce(const WalkArgs &a, WideSmem<T, ORDER, CONS> &P, unsigned &it,
+                                              bool &alive, volatile int *abort_flag,
                                               int32_t *stack, int stack_cap, int g, int gf,
-                                              int gn, const SysScalars &ss, float theta2,
+                                              int gn, const SysScalars &ss, T theta2,
                                               WalkCounters &wc) {
-  using T = float;
+  constexpr unsigned kSlots = WideSmem<T, ORDER, CONS>::kSlots;
+  const int lane = threadIdx.x & (kWarp - 1);
+  double gc[3];
+  int first = 1;
+  auto emit = [&](int kind, int count, const int *ids) {
+    const unsigned slot = it % kSlots, round = it / kSlots;
+    if (alive && round > 0 && !mbar_wait_warp(&P.empty[slot], (round - 1) & 1u, abort_flag))
+      alive = false;
+    if (!alive) return;
+    WideSlot &R = P.ring[slot];
+    if (lane < count) R.id[lane] = ids[lane];
+    if (lane == 0) {
+      R.kind = kind; R.count = count; R.g = g; R.first = first;
+      R.gc[0] = gc[0]; R.gc[1] = gc[1]; R.gc[2] = gc[2];
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&P.full[slot]);
+    ++it;
+    first = 0;
+  };
+  walk_members<T, ORDER, TPL, true>(
+      a, P.walk, stack, stack_cap, gf, gn, ss, theta2, gc, wc,
+      [](const T (&)[TPL], const T (&)[TPL], const T (&)[TPL]) {},
+      [&](int end, int nc) {
+        emit(kRingCells, nc, P.walk.cellq + end - nc);
+        wc.pc += (unsigned long long)nc * gn;
+      },
+      [&](int end, int nb) {
+        emit(kRingBodies, nb, P.walk.bodyq + end - nb);
+        wc.pp += (unsigned long long)nb * gn;
+      });
+  emit(kRingEnd, 0, P.walk.cellq);
+}
+
+// One slot of a group on its consumer: the batch's sums, then the turn.
+// False when a wait gave up.
+template <typename T, int ORDER, int TPL, bool SOFT, int CONS>
+__device__ __forceinline__ bool consume_slot(const WalkArgs &a, WideSmem<T, ORDER, CONS> &P, T *stage,
+                                             unsigned it, volatile int *abort_flag, int kind,
+                                             int count, int first, int id, int gf, int gn,
+                                             const double gc[3], const SysScalars &ss,
+                                             const Targets<T, TPL> &tg, double inv_s, T eps2) {
+  constexpr unsigned kSlots = WideSmem<T, ORDER, CONS>::kSlots;
+  const int lane = threadIdx.x & (kWarp - 1);
+  T sx[TPL], sy[TPL], sz[TPL];
+  if (kind == kRingCells) {
+    const double inv_m = 1.0 / ss.mass, nq = inv_m * inv_s * inv_s, no = nq * inv_s;
+    stage_cells<T, ORDER>(stage, lane, count, id, a, gc, inv_s, inv_m, nq, no);
+    __syncwarp();
+    sum_cells<T, ORDER, TPL>(stage, count, tg, eps2, sx, sy, sz);
+  } else if (kind == kRingBodies) {
+    const double inv_m = 1.0 / ss.mass;
+    stage_bodies<T>(stage, lane, count, id, a, gc, inv_s, inv_m);
+    __syncwarp();
+    sum_bodies<T, TPL, SOFT>(stage, count, tg, eps2, sx, sy, sz);
+  }
+  const unsigned slot = it % kSlots, round = it / kSlots;
+  if (!mbar_wait_warp(&P.turn[slot], round & 1u, abort_flag)) return false;
+  Sums<T, TPL> acc;
+  if (first) acc.clear();
+  else {
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      const int k = lane + kWarp * t;
+      acc.ax[t] = P.sums[0][k]; acc.ay[t] = P.sums[1][k]; acc.az[t] = P.sums[2][k];
+      if (acc.kKahan) { acc.cx[t] = P.sums[3][k]; acc.cy[t] = P.sums[4][k]; acc.cz[t] = P.sums[5][k]; }
+    }
+  }
+  if (kind != kRingEnd) {
+    acc.add(sx, sy, sz);
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      const int k = lane + kWarp * t;
+      P.sums[0][k] = acc.ax[t]; P.sums[1][k] = acc.ay[t]; P.sums[2][k] = acc.az[t];
+      if (acc.kKahan) { P.sums[3][k] = acc.cx[t]; P.sums[4][k] = acc.cy[t]; P.sums[5][k] = acc.cz[t]; }
+    }
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&P.turn[(it + 1) % kSlots]);
+  if (kind == kRingEnd) acc.write(a, ss, gf, gn, lane);
+  return true;
+}
+
+template <int CONS> constexpr int wide_threads() { return (1 + CONS) * kWarp; }
+// resident blocks per SM the kernel is compiled for: 16 warps of 128 registers
+template <int CONS> constexpr int wide_blocks() { return 16 / (1 + CONS); }
+
+template <typename T, int ORDER, int MAXTPL, bool SOFT, int CONS>
+__global__ void __launch_bounds__(wide_threads<CONS>(), wide_blocks<CONS>())
+wide_walk_kernel(WalkArgs a) {
+  extern __shared__ __align__(16) unsigned char wide_smem_raw[];
+  constexpr unsigned kSlots = WideSmem<T, ORDER, CONS>::kSlots;
+  WideSmem<T, ORDER, CONS> &P = *reinterpret_cast<WideSmem<T, ORDER, CONS> *>(wide_smem_raw);
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x & (kWarp - 1);
+  if (threadIdx.x == 0) {
+    for (unsigned r = 0; r < kSlots; ++r) {
+      mbar_init(&P.full[r], 1);
+      mbar_init(&P.empty[r], 1);
+      mbar_init(&P.turn[r], 1);
+    }
+    P.abort_flag = 0;
+    mbar_arrive(&P.turn[0]);  // the first batch has nobody before it
+  }
+  __syncthreads();
+  volatile int *abort_flag = &P.abort_flag;
+  if (warp == 0) {
+    const int ngroups = a.g_end >= 0 ? min(a.g_end, a.sc->n_groups) : a.sc->n_groups;
+    int32_t *stack = a.stack + (int64_t)blockIdx.x * a.stack_cap;
+    const int stack_cap = (int)a.stack_cap;
+    const T theta2 = (T)a.theta2;
+    WalkCounters wc;
+    bool alive = true;
+    unsigned it = 0;
+    for (;;) {
+      int g = 0;
+      if (lane == 0) g = a.g_begin + atomicAdd(a.cursor, 1);
+      g = __shfl_sync(kFull, g, 0);
+      if (g >= ngroups) break;
+      const int gf = a.g_first[g];
+      const int gn = a.g_first[g + 1] - gf;
+      const SysScalars &ss = a.ss[a.sys_of[gf]];
+      if (MAXTPL == 2 && gn > kWarp)
+        wide_produce<T, ORDER, 2, CONS>(a, P, it, alive, abort_flag, stack, stack_cap, g, gf, gn, ss,
+                                   theta2, wc);
+      else
+        wide_produce<T, ORDER, 1, CONS>(a, P, it, alive, abort_flag, stack, stack_cap, g, gf, gn, ss,
+                                   theta2, wc);
+      if (!alive) break;
+    }
+    // tell every consumer there is nothing more
+    for (int c = 0; alive && c < CONS; ++c, ++it) {
+      const unsigned slot = it % kSlots, round = it / kSlots;
+      if (round > 0 && !mbar_wait_warp(&P.empty[slot], (round - 1) & 1u, abort_flag)) {
+        alive = false;
+        break;
+      }
+      if (lane == 0) { P.ring[slot].kind = kRingQuit; mbar_arrive(&P.full[slot]); }
+    }
+    if (lane == 0) {
+      if (wc.err) atomicOr(&a.sc->err, wc.err);
+      if (!alive) atomicOr(&a.sc->err, kErrTimeout);
+      if (a.count_stats) {
+        atomicAdd(&a.stats[0], wc.pp);
+        atomicAdd(&a.stats[1], wc.pc);
+        atomicAdd(&a.stats[3], wc.tests);
+      }
+    }
+  } else {
+    T *stage = P.stage[warp - 1];
+    int cur = -1, gf = 0, gn = 0;
+    double gc[3] = {0.0, 0.0, 0.0}, inv_s = 0.0;
+    T eps2 = (T)0;
+    const SysScalars *ss = a.ss;
+    Targets<T, MAXTPL> tg;
+    bool ok = true;
+    for (unsigned it = warp - 1;; it += CONS) {
+      const unsigned slot = it % kSlots, round = it / kSlots;
+      ok = mbar_wait_warp(&P.full[slot], round & 1u, abort_flag);
+      if (!ok) break;
+      const WideSlot &R = P.ring[slot];
+      const int kind = R.kind, count = R.count, g = R.g, first = R.first, id = R.id[lane];
+      if (kind == kRingQuit) break;
+      if (g != cur) {  // the group's targets
+        cur = g;
+        gc[0] = R.gc[0]; gc[1] = R.gc[1]; gc[2] = R.gc[2];
+        gf = a.g_first[g];
+        gn = a.g_first[g + 1] - gf;
+        ss = a.ss + a.sys_of[gf];
+        inv_s = 1.0 / ss->ssa;
+        eps2 = group_eps2<T>(a, inv_s);
+#pragma unroll
+        for (int t = 0; t < MAXTPL; ++t) {
+          const int k = lane + kWarp * t;
+          const double4 p = a.spos[gf + (k < gn ? k : 0)];
+          tg.set(t, (T)((p.x - gc[0]) * inv_s), (T)((p.y - gc[1]) * inv_s),
+                 (T)((p.z - gc[2]) * inv_s));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&P.empty[slot]);
+      if (MAXTPL == 2 && gn > kWarp) {
+        ok = consume_slot<T, ORDER, MAXTPL, SOFT, CONS>(a, P, stage, it, abort_flag, kind, count, first,
+                                                  id, gf, gn, gc, *ss, tg, inv_s, eps2);
+      } else {
+        Targets<T, 1> t1;
+        t1.x[0] = tg.x[0]; t1.y[0] = tg.y[0]; t1.z[0] = tg.z[0];
+        ok = consume_slot<T, ORDER, 1, SOFT, CONS>(a, P, stage, it, abort_flag, kind, count, first, id,
+                                             gf, gn, gc, *ss, t1, inv_s, eps2);
+      }
+      if (!ok) break;
+    }
+    if (!ok && lane == 0) atomicOr(&a.sc->err, kErrTimeout);
+  }
+}
+
+// ---- warp-specialised FP32 walk for many groups ----
+//
+// A block holds kTeams teams of one producer warp and one consumer warp.  The
+// producer walks groups from the global cursor and stages every batch of 32
+// cells or bodies into a ring of kRing shared-memory slots; its consumer sums
+// the batches and writes the forces: the batches, order and arithmetic of the
+// one-warp walk, so the same bits.  The consumers (warpgroup 0) take registers
+// over from the producers (warpgroup 1) with setmaxnreg.
+// Bound: the FP32 FMA pipe (64 % busy at 2^20 bodies; the evaluation loop alone
+// reaches 84 % with 2-5 warps per scheduler, and the producers' instructions
+// take the difference).  2^20 Hernquist bodies 5.20 -> 5.17 ms, 5,000,011 in a
+// uniform sphere 7.00 -> 6.76 ms with the walk's gathered candidates and
+// shared-memory stack; consumers as the lower warpgroup took 1.3 % off.  Tried
+// and slower at 2^20: two batches at once, one per half-warp with four targets a
+// lane (2 blocks per SM: 7.1 ms), the consumers staging (7.0-9.0 ms), eight lanes
+// per opened node instead of the scan (5.47 ms), branches instead of the
+// predicated appends (5.45 ms).
+
+constexpr int kTeams = 4;
+constexpr int kRing = 4;
+
+template <int ORDER>
+struct __align__(16) TeamSlot {
+  int kind, count, g, unused;
+  double gc[3];
+  double unused2;
+  float stage[kWarp * StageWords<ORDER>::value];
+};
+
+template <int ORDER>
+struct __align__(16) TeamSmem {
+  unsigned long long full[kTeams][kRing];
+  unsigned long long empty[kTeams][kRing];
+  int abort_flag;
+  WalkSmem<float> walk[kTeams];
+  TeamSlot<ORDER> ring[kTeams][kRing];
+};
+
+// Producer side of one group: the walk of walk_group, with every batch staged
+// into the ring.  `alive` turns false (for the rest of the kernel) when a wait
+// gave up.
+template <int ORDER, int TPL>
+__device__ __forceinline__ void team_produce(const WalkArgs &a, TeamSmem<ORDER> &P, int team,
+                                             unsigned &it, bool &alive, volatile int *abort_flag,
+                                             int32_t *stack, int stack_cap, int g, int gf, int gn,
+                                             const SysScalars &ss, float theta2, WalkCounters &wc) {
   const double inv_s = 1.0 / ss.ssa, inv_m = 1.0 / ss.mass;
   const double nq = inv_m * inv_s * inv_s, no = nq * inv_s;
-  constexpr int W = StageWords<ORDER>::value;
   const int lane = threadIdx.x & (kWarp - 1);
-  double px[TPL], py[TPL], pz[TPL];
+  double gc[3];
+  // the next slot, once its consumer has released it
+  auto acquire = [&]() -> TeamSlot<ORDER> & {
+    const unsigned slot = it % kRing, round = it / kRing;
+    if (alive && round > 0 && !mbar_wait_warp(&P.empty[team][slot], (round - 1) & 1u, abort_flag))
+      alive = false;
+    return P.ring[team][slot];
+  };
+  auto publish = [&]() {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&P.full[team][it % kRing]);
+    ++it;
+  };
+  walk_members<float, ORDER, TPL, false>(
+      a, P.walk[team], stack, stack_cap, gf, gn, ss, theta2, gc, wc,
+      [&](const float (&)[TPL], const float (&)[TPL], const float (&)[TPL]) {
+        TeamSlot<ORDER> &R = acquire();
+        if (!alive) return;
+        if (lane == 0) {
+          R.kind = kRingStart; R.g = g; R.count = gn;
+          R.gc[0] = gc[0]; R.gc[1] = gc[1]; R.gc[2] = gc[2];
+        }
+        publish();
+      },
+      [&](int end, int nc) {
+        TeamSlot<ORDER> &R = acquire();
+        if (!alive) return;
+        stage_cells<float, ORDER>(R.stage, lane, nc,
+                                  lane < nc ? P.walk[team].cellq[end - nc + lane] : 0, a, gc, inv_s,
+                                  inv_m, nq, no);
+        if (lane == 0) { R.kind = kRingCells; R.count = nc; }
+        wc.pc += (unsigned long long)nc * gn;
+        publish();
+      },
+      [&](int end, int nb) {
+        TeamSlot<ORDER> &R = acquire();
+        if (!alive) return;
+        stage_bodies<float>(R.stage, lane, nb, lane < nb ? P.walk[team].bodyq[end - nb + lane] : 0,
+                            a, gc, inv_s, inv_m);
+        if (lane == 0) { R.kind = kRingBodies; R.count = nb; }
+        wc.pp += (unsigned long long)nb * gn;
+        publish();
+      });
+  TeamSlot<ORDER> &R = acquire();
+  if (!alive) return;
+  if (lane == 0) R.kind = kRingEnd;
+  publish();
+}
+
+// Consumer side of one group (its start slot already read and released):
+// sums the batches until the group's end slot, then writes the forces; false
+// when a wait gave up.
+template <int ORDER, int TPL, bool SOFT>
+__device__ __forceinline__ bool team_consume(const WalkArgs &a, TeamSmem<ORDER> &P, int team,
+                                             unsigned &it, volatile int *abort_flag, int gf, int gn,
+                                             const double gc[3], const SysScalars &ss) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const double inv_s = 1.0 / ss.ssa;
+  const float eps2 = group_eps2<float>(a, inv_s);
+  Targets<float, TPL> tg;
 #pragma unroll
   for (int t = 0; t < TPL; ++t) {
     const int k = lane + kWarp * t;
     const double4 p = a.spos[gf + (k < gn ? k : 0)];
-    px[t] = p.x; py[t] = p.y; pz[t] = p.z;
+    tg.set(t, (float)((p.x - gc[0]) * inv_s), (float)((p.y - gc[1]) * inv_s),
+           (float)((p.z - gc[2]) * inv_s));
   }
-  double lo[3] = {px[0], py[0], pz[0]}, hi[3] = {px[0], py[0], pz[0]};
-#pragma unroll
-  for (int t = 1; t < TPL; ++t) {
-    lo[0] = fmin(lo[0], px[t]); hi[0] = fmax(hi[0], px[t]);
-    lo[1] = fmin(lo[1], py[t]); hi[1] = fmax(hi[1], py[t]);
-    lo[2] = fmin(lo[2], pz[t]); hi[2] = fmax(hi[2], pz[t]);
-  }
-  double gc[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) gc[k] = 0.5 * (warp_min(lo[k]) + warp_max(hi[k]));
-  T rx[TPL], ry[TPL], rz[TPL], blo[3], bhi[3];
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    rx[t] = (T)((px[t] - gc[0]) * inv_s);
-    ry[t] = (T)((py[t] - gc[1]) * inv_s);
-    rz[t] = (T)((pz[t] - gc[2]) * inv_s);
-    if (t == 0) { blo[0] = bhi[0] = rx[0]; blo[1] = bhi[1] = ry[0]; blo[2] = bhi[2] = rz[0]; }
-    else {
-      blo[0] = min(blo[0], rx[t]); bhi[0] = max(bhi[0], rx[t]);
-      blo[1] = min(blo[1], ry[t]); bhi[1] = max(bhi[1], ry[t]);
-      blo[2] = min(blo[2], rz[t]); bhi[2] = max(bhi[2], rz[t]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) { blo[k] = warp_min(blo[k]); bhi[k] = warp_max(bhi[k]); }
-  const T diag = sqrt((bhi[0] - blo[0]) * (bhi[0] - blo[0]) + (bhi[1] - blo[1]) * (bhi[1] - blo[1]) +
-                      (bhi[2] - blo[2]) * (bhi[2] - blo[2]));
-  const T inv_theta2 = theta2 > (T)0 ? (T)1 / theta2 : (T)INFINITY;
-  T rad2 = (T)0;
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) rad2 = max(rad2, fma(rx[t], rx[t], fma(ry[t], ry[t], rz[t] * rz[t])));
-  const T rad = sqrt(warp_max(rad2));
-
-  // the next slot, once its consumer has released it
-  auto acquire = [&]() -> RingSlot<ORDER> * {
-    const int slot = it % kRing;
-    const unsigned round = (unsigned)(it / kRing);
-    if (alive && round > 0 && !mbar_wait_warp(&P.empty[team][slot], (round - 1) & 1u, abort_flag))
-      alive = false;
-    return &P.ring[team][slot];
-  };
-  auto publish = [&]() {
-    __syncwarp();
-    mbar_arrive(&P.full[team][it % kRing]);
-    ++it;
-  };
-  RingSlot<ORDER> *R = acquire();
-  if (alive) {
-    if (lane == 0) {
-      R->kind = kRingStart; R->g = g; R->count = gn;
-      R->gc[0] = gc[0]; R->gc[1] = gc[1]; R->gc[2] = gc[2];
-    }
-    publish();
-  }
-  // the stage layouts of walk_group's paired evaluation
-  auto emit_cells = [&](int end, int nc) {
-    RingSlot<ORDER> *Q = acquire();
-    if (!alive) return;
-    float *w = Q->stage + (lane >> 1) * 2 * W + (lane & 1);
-    if (lane < nc) {
-      stage_cell<float, ORDER, 2>(w, P.cellq[team][end - nc + lane], a, gc, inv_s, inv_m, nq, no);
-    } else if (lane == nc && (nc & 1)) {
-#pragma unroll
-      for (int k = 3; k < W; ++k) w[2 * k] = 0.0f;
-      w[0] = w[2] = w[4] = kPadPos;
-    }
-    if (lane == 0) { Q->kind = kRingCells; Q->count = nc; }
-    wc.pc += (unsigned long long)nc * gn;
-    publish();
-  };
-  auto emit_bodies = [&](int end, int nb) {
-    RingSlot<ORDER> *Q = acquire();
-    if (!alive) return;
-    float *w = Q->stage + (lane >> 1) * 8 + (lane & 1);
-    if (lane < nb) {
-      const int p = P.bodyq[team][end - nb + lane];
-      const double4 sp = a.spos[p];
-      w[0] = (float)((sp.x - gc[0]) * inv_s);
-      w[2] = (float)((sp.y - gc[1]) * inv_s);
-      w[4] = (float)((sp.z - gc[2]) * inv_s);
-      w[6] = (float)(sp.w * inv_m);
-    } else if (lane == nb && (nb & 1)) {
-      w[0] = w[2] = w[4] = kPadPos;
-      w[6] = 0.0f;
-    }
-    if (lane == 0) { Q->kind = kRingBodies; Q->count = nb; }
-    wc.pp += (unsigned long long)nb * gn;
-    publish();
-  };
-  tree_walk<T, TPL, bodies_as_cell<ORDER>()>(a, P.cellq[team], P.bodyq[team], stack, stack_cap, gf, gn, ss.root, gc, inv_s,
-                    blo, bhi, theta2, inv_theta2, diag, rad, rx, ry, rz, wc, emit_cells,
-                    emit_bodies);
-  R = acquire();
-  if (alive) {
-    if (lane == 0) R->kind = kRingEnd;
-    publish();
-  }
-}
-
-// Consumer side of one group (its start slot already read and released):
-// evaluates batches until the group's end slot, then writes the forces as
-// walk_group does; false when a wait gave up.
-template <int ORDER, int TPL, bool SOFT>
-__device__ __forceinline__ bool consume_group(const WalkArgs &a, PipeSmem<ORDER> &P, int team,
-                                              int &it, volatile int *abort_flag, int gf, int gn,
-                                              const double gc[3], const SysScalars &ss) {
-  using T = float;
-  constexpr int W = StageWords<ORDER>::value;
-  const int lane = threadIdx.x & (kWarp - 1);
-  const double inv_s = 1.0 / ss.ssa;
-  const T eps2 = (T)(a.eps2 * inv_s * inv_s);
-  const float2 eps2p = splat(eps2);
-  bool valid[TPL];
-  float2 nrx[TPL], nry[TPL], nrz[TPL];
-  T ax[TPL], ay[TPL], az[TPL], cx[TPL], cy[TPL], cz[TPL];
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    const int k = lane + kWarp * t;
-    valid[t] = k < gn;
-    const double4 p = a.spos[gf + (valid[t] ? k : 0)];
-    nrx[t] = splat(-(T)((p.x - gc[0]) * inv_s));
-    nry[t] = splat(-(T)((p.y - gc[1]) * inv_s));
-    nrz[t] = splat(-(T)((p.z - gc[2]) * inv_s));
-    ax[t] = ay[t] = az[t] = cx[t] = cy[t] = cz[t] = (T)0;
-  }
+  Sums<float, TPL> acc;
+  acc.clear();
   for (;;) {
-    const int slot = it % kRing;
-    const unsigned round = (unsigned)(it / kRing);
+    const unsigned slot = it % kRing, round = it / kRing;
     if (!mbar_wait_warp(&P.full[team][slot], round & 1u, abort_flag)) return false;
-    const RingSlot<ORDER> &R = P.ring[team][slot];
-    const int kind = R.kind, cnt = R.count;
+    const TeamSlot<ORDER> &R = P.ring[team][slot];
+    const int kind = R.kind, count = R.count;
+    float sx[TPL], sy[TPL], sz[TPL];
     if (kind == kRingCells) {
-      float2 bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
-      const int np = (cnt + 1) >> 1;
-#pragma unroll 2
-      for (int j = 0; j < np; ++j) {
-        const float4 *st = reinterpret_cast<const float4 *>(R.stage) + j * (W / 2);
-        float2 cw[W];
-#pragma unroll
-        for (int k = 0; k < W / 2; ++k) {
-          const float4 v = st[k];
-          cw[2 * k] = make_float2(v.x, v.y);
-          cw[2 * k + 1] = make_float2(v.z, v.w);
-        }
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-          cell_force2<ORDER>(cw, nrx[t], nry[t], nrz[t], eps2p, bx[t], by[t], bz[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        kahan_add(ax[t], cx[t], bx[t].x + bx[t].y);
-        kahan_add(ay[t], cy[t], by[t].x + by[t].y);
-        kahan_add(az[t], cz[t], bz[t].x + bz[t].y);
-      }
+      sum_cells<float, ORDER, TPL>(R.stage, count, tg, eps2, sx, sy, sz);
+      acc.add(sx, sy, sz);
     } else if (kind == kRingBodies) {
-      float2 bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) bx[t] = by[t] = bz[t] = make_float2(0.0f, 0.0f);
-      const int np = (cnt + 1) >> 1;
-      const float4 *st = reinterpret_cast<const float4 *>(R.stage);
-      for (int j = 0; j < np; ++j) {
-        const float4 u = st[2 * j], v = st[2 * j + 1];
-        const float2 sx = make_float2(u.x, u.y), sy = make_float2(u.z, u.w);
-        const float2 sz = make_float2(v.x, v.y), sm = make_float2(v.z, v.w);
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-          body_force2<SOFT>(sx, sy, sz, sm, nrx[t], nry[t], nrz[t], eps2p, bx[t], by[t], bz[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        kahan_add(ax[t], cx[t], bx[t].x + bx[t].y);
-        kahan_add(ay[t], cy[t], by[t].x + by[t].y);
-        kahan_add(az[t], cz[t], bz[t].x + bz[t].y);
-      }
+      sum_bodies<float, TPL, SOFT>(R.stage, count, tg, eps2, sx, sy, sz);
+      acc.add(sx, sy, sz);
     }
     __syncwarp();
-    mbar_arrive(&P.empty[team][slot]);
+    if (lane == 0) mbar_arrive(&P.empty[team][slot]);
     ++it;
     if (kind == kRingEnd) break;
   }
-  const double scale = a.G * ss.mass * inv_s * inv_s;
-  double *out = a.out + 3 * ss.off;
-  const int64_t ns = ss.n;
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    if (!valid[t]) continue;
-    const int i = gf + lane + kWarp * t;
-    const int64_t p = a.perm[i] - ss.off;
-    double fxs = (double)ax[t], fys = (double)ay[t], fzs = (double)az[t];
-    fxs -= (double)cx[t]; fys -= (double)cy[t]; fzs -= (double)cz[t];
-    double sc = scale;
-    if (a.out_kind == 0) sc *= a.spos[i].w;
-    out[p] = fxs * sc;
-    out[ns + p] = fys * sc;
-    out[2 * ns + p] = fzs * sc;
-  }
+  acc.write(a, ss, gf, gn, lane);
   return true;
 }
 
-// PipeRegs<ORDER>::blocks blocks of 2 kTeams warps per SM.  At launch every
+// TeamRegs<ORDER>::blocks blocks of 2 kTeams warps per SM.  At launch every
 // thread holds `regs` registers (the most that `blocks` blocks allow); the
 // producer warpgroup then gives registers up to the consumer warpgroup:
 // producer + consumer = 2 regs, so the consumers' request is always covered by
-// the block's own registers (the host checks the launch count first).  The
-// quadrupole consumer runs without spills at 96, the octupole one needs more.
-constexpr int kPipeThreads = 2 * kTeams * kWarp;
+// the block's own registers (the host checks the launch count first).
+constexpr int kTeamThreads = 2 * kTeams * kWarp;
 static_assert(kTeams == 4, "one warpgroup of producers, one of consumers");
-template <int ORDER> struct PipeRegs {
+template <int ORDER> struct TeamRegs {
   static constexpr int blocks = ORDER >= 8 ? 2 : 3;
   static constexpr int regs = ORDER >= 8 ? 128 : 80;
   static constexpr int producer = ORDER >= 8 ? 96 : 64;
   static constexpr int consumer = 2 * regs - producer;
-  static_assert(regs * kPipeThreads * blocks <= 65536, "register file");
+  static_assert(regs * kTeamThreads * blocks <= 65536, "register file");
   static_assert(regs % 8 == 0 && producer % 8 == 0 && consumer <= 256, "setmaxnreg counts");
 };
 
 template <int ORDER, int MAXTPL, bool SOFT>
-__global__ void __launch_bounds__(kPipeThreads, PipeRegs<ORDER>::blocks)
-pipe_walk_kernel(WalkArgs a) {
-  extern __shared__ __align__(16) unsigned char pipe_smem_raw[];
-  PipeSmem<ORDER> &P = *reinterpret_cast<PipeSmem<ORDER> *>(pipe_smem_raw);
+__global__ void __launch_bounds__(kTeamThreads, TeamRegs<ORDER>::blocks)
+team_walk_kernel(WalkArgs a) {
+  extern __shared__ __align__(16) unsigned char team_smem_raw[];
+  TeamSmem<ORDER> &P = *reinterpret_cast<TeamSmem<ORDER> *>(team_smem_raw);
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x & (kWarp - 1);
   if (threadIdx.x == 0) {
     for (int q = 0; q < kTeams; ++q)
       for (int r = 0; r < kRing; ++r) {
-        mbar_init(&P.full[q][r], kWarp);
-        mbar_init(&P.empty[q][r], kWarp);
+        mbar_init(&P.full[q][r], 1);
+        mbar_init(&P.empty[q][r], 1);
       }
     P.abort_flag = 0;
   }
   __syncthreads();
   volatile int *abort_flag = &P.abort_flag;
-  const int ngroups = a.g_end >= 0 ? min(a.g_end, a.sc->n_groups) : a.sc->n_groups;
-  int it = 0;
-  if (warp < kTeams) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PipeRegs<ORDER>::producer));
-    const int team = warp;
+  unsigned it = 0;
+  if (warp >= kTeams) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TeamRegs<ORDER>::producer));
+    const int ngroups = a.g_end >= 0 ? min(a.g_end, a.sc->n_groups) : a.sc->n_groups;
+    const int team = warp - kTeams;
     int32_t *stack = a.stack + ((int64_t)blockIdx.x * kTeams + team) * a.stack_cap;
     const int stack_cap = (int)a.stack_cap;
     const float theta2 = (float)a.theta2;
@@ -1145,20 +1441,19 @@ pipe_walk_kernel(WalkArgs a) {
       const int gn = a.g_first[g + 1] - gf;
       const SysScalars &ss = a.ss[a.sys_of[gf]];
       if (MAXTPL == 2 && gn > kWarp)
-        produce_group<ORDER, 2, SOFT>(a, P, team, it, alive, abort_flag, stack, stack_cap, g, gf,
-                                      gn, ss, theta2, wc);
+        team_produce<ORDER, 2>(a, P, team, it, alive, abort_flag, stack, stack_cap, g, gf, gn, ss,
+                               theta2, wc);
       else
-        produce_group<ORDER, 1, SOFT>(a, P, team, it, alive, abort_flag, stack, stack_cap, g, gf,
-                                      gn, ss, theta2, wc);
+        team_produce<ORDER, 1>(a, P, team, it, alive, abort_flag, stack, stack_cap, g, gf, gn, ss,
+                               theta2, wc);
       if (!alive) break;
     }
     if (alive) {  // tell the consumer there is nothing more
-      const int slot = it % kRing;
-      const unsigned round = (unsigned)(it / kRing);
+      const unsigned slot = it % kRing, round = it / kRing;
       if (round == 0 || mbar_wait_warp(&P.empty[team][slot], (round - 1) & 1u, abort_flag)) {
-        if (lane == 0) P.ring[team][slot].kind = kRingQuit;
-        __syncwarp();
-        mbar_arrive(&P.full[team][slot]);
+        if (lane == 0) { P.ring[team][slot].kind = kRingQuit; mbar_arrive(&P.full[team][slot]); }
+      } else {
+        alive = false;
       }
     }
     if (lane == 0) {
@@ -1171,34 +1466,28 @@ pipe_walk_kernel(WalkArgs a) {
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PipeRegs<ORDER>::consumer));
-    const int team = warp - kTeams;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TeamRegs<ORDER>::consumer));
+    const int team = warp;
+    bool ok;
     for (;;) {
-      const int slot = it % kRing;
-      const unsigned round = (unsigned)(it / kRing);
-      if (!mbar_wait_warp(&P.full[team][slot], round & 1u, abort_flag)) {
-        if (lane == 0) atomicOr(&a.sc->err, kErrTimeout);
-        break;
-      }
-      const RingSlot<ORDER> &R = P.ring[team][slot];
+      ok = mbar_wait_warp(&P.full[team][it % kRing], (it / kRing) & 1u, abort_flag);
+      if (!ok) break;
+      const TeamSlot<ORDER> &R = P.ring[team][it % kRing];
       const int kind = R.kind, g = R.g, gn = R.count;
       const double gc[3] = {R.gc[0], R.gc[1], R.gc[2]};
-      __syncwarp();
-      mbar_arrive(&P.empty[team][slot]);
-      ++it;
       if (kind != kRingStart) break;  // the producer has no more groups
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&P.empty[team][it % kRing]);
+      ++it;
       const int gf = a.g_first[g];
       const SysScalars &ss = a.ss[a.sys_of[gf]];
-      bool ok;
       if (MAXTPL == 2 && gn > kWarp)
-        ok = consume_group<ORDER, 2, SOFT>(a, P, team, it, abort_flag, gf, gn, gc, ss);
+        ok = team_consume<ORDER, 2, SOFT>(a, P, team, it, abort_flag, gf, gn, gc, ss);
       else
-        ok = consume_group<ORDER, 1, SOFT>(a, P, team, it, abort_flag, gf, gn, gc, ss);
-      if (!ok) {
-        if (lane == 0) atomicOr(&a.sc->err, kErrTimeout);
-        break;
-      }
+        ok = team_consume<ORDER, 1, SOFT>(a, P, team, it, abort_flag, gf, gn, gc, ss);
+      if (!ok) break;
     }
+    if (!ok && lane == 0) atomicOr(&a.sc->err, kErrTimeout);
   }
 }
 
@@ -1425,53 +1714,95 @@ int probe_bounded_wait(long long cycles, long long *out5) {
   return rc;
 }
 
-// The pipelined walk, when the kernel was built with the register count its
-// setmaxnreg split assumes; returns false (nothing launched) otherwise.
-template <int ORDER, int MAXTPL, bool SOFT>
-static bool launch_pipe_walk(const WalkArgs &a, cudaStream_t s) {
-  // the shared-memory limit is a per-device attribute: set it once per device
-  static int per_sm[64] = {};
-  const int smem = (int)sizeof(PipeSmem<ORDER>);
+// exactly the blocks that are resident at once: no block waits for a second
+// wave behind the walk (which would also hold back other streams); occupancy
+// and the shared-memory limit are properties of the device, so they are kept
+// per device.  regs > 0: the kernel's setmaxnreg split assumes that launch
+// count; a block launched with fewer would wait for ever, so a kernel compiled
+// otherwise is never launched (-1).
+template <typename K>
+static int resident_blocks(int (&per_sm)[64], K *kernel, int threads, size_t smem, int regs = 0) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   if (per_sm[dev] == 0) {
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, pipe_walk_kernel<ORDER, MAXTPL, SOFT>);
-    cudaFuncSetAttribute(pipe_walk_kernel<ORDER, MAXTPL, SOFT>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int v = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, pipe_walk_kernel<ORDER, MAXTPL, SOFT>,
-                                                  kPipeThreads, smem);
-    // a block launched with fewer registers than the split hands out would
-    // wait for ever in setmaxnreg.inc: never launch it
-    per_sm[dev] = (fa.numRegs == PipeRegs<ORDER>::regs && v > 0) ? v : -1;
+    if (smem)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, smem);
+    cudaFuncAttributes fa{};
+    cudaFuncGetAttributes(&fa, kernel);
+    per_sm[dev] = regs > 0 && (fa.numRegs != regs || v < 1) ? -1 : (v > 0 ? v : 1);
   }
-  if (per_sm[dev] < 0) return false;
-  int64_t blocks = (int64_t)per_sm[dev] * sm_count();
-  if (blocks * kTeams > a.slots) blocks = a.slots / kTeams;  // one stack per producer
-  pipe_walk_kernel<ORDER, MAXTPL, SOFT><<<(unsigned)blocks, kPipeThreads, smem, s>>>(a);
+  return per_sm[dev];
+}
+
+template <int ORDER, int MAXTPL, bool SOFT>
+static bool launch_team_walk(const WalkArgs &a, cudaStream_t s) {
+  static int per_sm[64] = {};
+  const size_t smem = sizeof(TeamSmem<ORDER>);
+  const int per = resident_blocks(per_sm, team_walk_kernel<ORDER, MAXTPL, SOFT>, kTeamThreads, smem,
+                                  TeamRegs<ORDER>::regs);
+  if (per < 0 || a.slots < kTeams) return false;
+  const int64_t blocks = bh_min64(a.slots / kTeams, (int64_t)sm_count() * per);  // a stack per producer
+  team_walk_kernel<ORDER, MAXTPL, SOFT><<<(unsigned)blocks, kTeamThreads, smem, s>>>(a);
   return true;
 }
 
+template <typename T, int ORDER, int MAXTPL, bool SOFT, int CONS>
+static void launch_wide_walk(const WalkArgs &a, cudaStream_t s) {
+  static int per_sm[64] = {};
+  const size_t smem = sizeof(WideSmem<T, ORDER, CONS>);
+  const int per = resident_blocks(per_sm, wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS>,
+                                  wide_threads<CONS>(), smem);
+  const int64_t blocks = bh_min64(a.slots, (int64_t)sm_count() * per);  // one stack per block
+  wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS><<<(unsigned)blocks, wide_threads<CONS>(), smem, s>>>(a);
+}
+
+// Which walk a launch takes (pipeline 1).  Few groups leave most of the chip
+// idle, so the more warps share a group the better, until the producers fall
+// short; a team's two warps per group fill the chip from about 1,000 groups on.
+// Walk times in us, 7 consumers / 3 consumers / teams (theta 0.5, Plummer):
+//   quadrupole  16,384: 157 / 189 / 371   24,000: 233 / 214 / 420
+//               65,536: 579 / 444 / 516  100,003: 865 / 671 / 549
+//   monopole    16,384: 148 / 159 / 259   65,536: 544 / 350 / 326
+//   octupole    16,384: 235 / 381 / 491   49,152: 682 / 730 / 707
+//               65,536: 925 / 965 / 788
+//   FP64 quad   16,384: 207 / 317 / -     24,000: 301 / 338 / -
+//               32,768: 375 / 374 / -    100,003: 1095 / 1048 / -
+//   FP64 oct    16,384: 398 / 666 / -    100,003: 2257 / 2363 / -
+// (uniform spheres cross at the same sizes within a third).  The octupole, whose
+// batches take longest, never does better with 3 consumers.
+template <typename T, int ORDER> constexpr int64_t seven_max() {
+  return ORDER >= 8 ? INT64_MAX : (sizeof(T) == 8 ? 24576 : 20480);
+}
+template <int ORDER> constexpr int64_t team_min() { return ORDER >= 8 ? 49153 : 65537; }
+// Above this the FP64 walk goes back to one warp per group, whose 16 groups per
+// SM keep the FP64 pipe fuller (theta 0.4, Hernquist, wide / one warp, us):
+//   monopole 131,072: 1504 / 1645  190,000: 2184 / 2196  262,144: 3075 / 2876
+//   quad     190,000: 3296 / 3566  262,144: 4579 / 4711  2^20 (theta 0.5): 11697 / 10338
+//   octupole 131,072: 5220 / 5859  190,000: 7756 / 7832  262,144: 10914 / 10536
+template <int ORDER> constexpr int64_t wide64_max() { return ORDER == 4 ? 262144 : 196608; }
+
+
 template <typename T, int ORDER, int MAXTPL, bool SOFT>
 static void launch_group_walk(const WalkArgs &a, cudaStream_t s) {
-  if (sizeof(T) == 4 && a.pipeline && launch_pipe_walk<ORDER, MAXTPL, SOFT>(a, s)) return;
-  // exactly the blocks that are resident at once: no block waits for a
-  // second wave behind the walk (which would also hold back other streams);
-  // occupancy is a property of the device, so it is kept per device
-  static int per_sm[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (per_sm[dev] == 0) {
-    int v = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, group_walk_kernel<T, ORDER, MAXTPL, SOFT>,
-                                                  kWarp, 0);
-    per_sm[dev] = v > 0 ? v : 1;
+  if (a.pipeline && (sizeof(T) == 4 || a.n <= wide64_max<ORDER>())) {
+    if constexpr (sizeof(T) == 4) {
+      if (a.n >= team_min<ORDER>() && launch_team_walk<ORDER, MAXTPL, SOFT>(a, s)) return;
+    }
+    if constexpr (ORDER < 8) {
+      if (a.n > seven_max<T, ORDER>()) {
+        launch_wide_walk<T, ORDER, MAXTPL, SOFT, 3>(a, s);
+        return;
+      }
+    }
+    launch_wide_walk<T, ORDER, MAXTPL, SOFT, 7>(a, s);
+    return;
   }
-  int64_t blocks = (int64_t)per_sm[dev] * sm_count();
-  if (blocks > a.slots) blocks = a.slots;
+  static int per_sm[64] = {};
+  const int per = resident_blocks(per_sm, group_walk_kernel<T, ORDER, MAXTPL, SOFT>, kWarp, 0);
+  const int64_t blocks = bh_min64(a.slots, (int64_t)sm_count() * per);  // one stack per block
   group_walk_kernel<T, ORDER, MAXTPL, SOFT><<<(unsigned)blocks, kWarp, 0, s>>>(a);
 }
 

@@ -68,10 +68,11 @@ typedef struct bh_params {
                          (octree_default.f90:1927-1936); 1 also accept a node that
                          fails it when it holds none of the group's bodies and passes
                          every group member's own MAC (morton_octree.f90:701-706)   */
-    int pipeline;     /* FP32 group walk: 0 one warp walks a group and evaluates it;
-                         1 producer warps walk the tree and stage the batches into a
-                         shared-memory ring, consumer warps evaluate them (the same
-                         results bit for bit; no reference counterpart)            */
+    int pipeline;     /* group walk: 0 one warp walks a group and evaluates it;
+                         1 producer warps walk the tree and hand the batches on
+                         through a shared-memory ring, consumer warps evaluate them
+                         (the same results bit for bit; no reference counterpart;
+                         large FP64 walks stay on one warp per group)              */
 } bh_params;
 
 /* Defaults: theta 0.5, G 1, eps 0, order 4, forces, depth 21, FP32, amp 1.2,

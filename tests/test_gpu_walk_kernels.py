@@ -1,0 +1,74 @@
+"""The walk kernels that a call's size chooses between give the bits of the
+one-warp walk (pipeline 0): the same batches, in the same order, with the same
+arithmetic.  Sizes lie on both sides of every switch, plus the smallest trees,
+groups of one target per lane, and shapes that fill the walk's queues: bodies
+with equal keys (ranges above 16 bodies), large leaves, a wide shallow tree and
+a deep one whose stack leaves its shared-memory window."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _forces(m, q, **kw):
+    from hierarquicos_b200.system import BHSystem
+
+    s = BHSystem()
+    f = s.forces(m, q[:, 0], q[:, 1], q[:, 2], **kw).cpu().numpy()
+    s.close()
+    return f
+
+
+def _same(m, q, **kw):
+    a, b = _forces(m, q, pipeline=0, **kw), _forces(m, q, pipeline=1, **kw)
+    assert np.isfinite(a).all()
+    assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
+
+
+def _cloud(n, seed, cusp=False):
+    rng = np.random.default_rng(seed)
+    q = rng.normal(size=(n, 3))
+    if cusp:
+        q *= rng.uniform(size=(n, 1)) ** 4
+    return rng.uniform(0.5, 1.5, n) / n, q
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("order", [1, 4, 8])
+@pytest.mark.parametrize("n", [1, 2, 33, 65, 1500])
+def test_small_trees(n, order, precision):
+    _same(*_cloud(n, n), order=order, precision=precision, theta=0.5, eps=0.01)
+
+
+@pytest.mark.parametrize("n,order,precision", [
+    (20480, 4, 0), (20481, 4, 0), (65536, 1, 0), (65537, 1, 0), (49152, 8, 0), (49153, 8, 0),
+    (24576, 4, 1), (24577, 1, 1), (196608, 1, 1), (196609, 8, 1), (262144, 4, 1), (262145, 4, 1)])
+def test_both_sides_of_a_switch(n, order, precision):
+    _same(*_cloud(n, 3), order=order, precision=precision, theta=0.8, eps=0.0)
+
+
+@pytest.mark.parametrize("n", [3000, 30000, 70000])
+@pytest.mark.parametrize("kw", [dict(group_size=32), dict(leaf_cap=64), dict(theta=0.15),
+                                dict(mac=0), dict(depth=4), dict(out_kind=1)])
+def test_shapes(n, kw):
+    kw = dict(dict(order=4, theta=0.6, eps=0.01), **kw)
+    if n > 30000 and kw["theta"] < 0.5:
+        n = 66000
+    _same(*_cloud(n, 7, cusp=True), **kw)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_equal_keys(precision):
+    """Buckets of 1..200 coincident bodies: leaf ranges of every length."""
+    rng = np.random.default_rng(11)
+    sizes = rng.integers(1, 200, 60)
+    q = np.repeat(rng.normal(size=(60, 3)), sizes, axis=0)
+    m = np.full(len(q), 1.0 / len(q))
+    _same(m, q, order=4, precision=precision, theta=0.5, eps=0.05)
+
+
+def test_softening_beyond_any_distance():
+    """FP64: eps^2 past the reciprocal series' range gives zero forces."""
+    m, q = _cloud(500, 1)
+    assert (_forces(m, q, order=4, precision=1, eps=1e160) == 0.0).all()
