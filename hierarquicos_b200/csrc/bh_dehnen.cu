@@ -314,8 +314,15 @@ dual_gen_kernel(Ent e, const int2 *__restrict__ fin, const unsigned long long *_
   __shared__ int ws[kGenWarps];
   __shared__ int s_tile;
   __shared__ int64_t s_base[2];
-  // after an overflow the count exceeds what was written: read only the buffer
-  const int64_t n_in = bh_min64((int64_t)*nin, cap_in);
+  // After a frontier overflow the count exceeds what was written and the buffer
+  // has slots that no pair was written to (any pair whose outputs did not fit):
+  // the later generations take nothing from it, and the host repeats the
+  // traversal with larger buffers.
+  // (one thread looks: another block may raise the flag meanwhile)
+  if (threadIdx.x == 0) s_tile = (int)(*(volatile unsigned long long *)flags & 1ull);
+  __syncthreads();
+  const int64_t n_in = s_tile ? 0 : bh_min64((int64_t)*nin, cap_in);
+  __syncthreads();
   const int64_t mut_base = (int64_t)*nmut_in;
   const int64_t ntiles = (n_in + kGenTile - 1) / kGenTile;
   if (ntiles == 0) {

@@ -183,3 +183,23 @@ def test_dehnen_refused_where_lists_cannot_be_sized(bh):
     rc = _lib.lib().bh_compute_forces_noalloc(dm.data_ptr(), dx.data_ptr(), dy.data_ptr(),
                                               dz.data_ptr(), 512, C.byref(p), out.data_ptr(), None)
     assert rc == _lib.BH_ERR_INVALID
+
+
+def test_dehnen_frontier_overflow_on_fresh_memory(bh):
+    """The first call of a handle outgrows its first pair buffers (this system's
+    frontier peaks at 18 pairs per body, the first buffer holds 16): whatever
+    the fresh memory held, the result is the second call's."""
+    import torch
+
+    m, q = plummer(3000, seed=4)
+    for word in (0x7FFFFFFF, -0x7FFFFFF0, 0x01234567):
+        fill = torch.full((1 << 26,), word, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        del fill
+        torch.cuda.empty_cache()
+        s = bh.BHSystem()
+        kw = dict(theta=0.5, eps=0.01, order=1, precision=3)
+        first = s.forces(m, *xyz(q), **kw).cpu().numpy()
+        again = s.forces(m, *xyz(q), **kw).cpu().numpy()
+        s.close()
+        assert np.isfinite(first).all() and np.array_equal(first, again)
