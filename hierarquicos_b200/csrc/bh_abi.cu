@@ -88,8 +88,8 @@ void drop_graph(bh_system *s) {
 
 void free_body_buffers(Buffers &b) {
   void *ptrs[] = {b.hm, b.hx, b.hy, b.hz, b.hout, b.k0, b.k1, b.v0, b.v1, b.hist, b.sys_of,
-                  b.spos, b.bn_left, b.bn_right, b.bn_parent, b.bn_first, b.bn_last, b.bn_level,
-                  b.bn_flag, b.bin2cn, b.cn_bin, b.cn_meta, b.cn_child, b.cn_parent, b.cn_com,
+                  b.spos, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
+                  b.bn_rank, b.up_list, b.cn_bin, b.cn_meta, b.cn_child, b.cn_parent, b.cn_com,
                   b.cn_quad, b.cn_oct, b.cn_fq, b.cn_fo, b.gflag, b.gscan, b.g_first, b.scan_tmp};
   for (void *q : ptrs)
     if (q) cudaFree(q);
@@ -97,8 +97,8 @@ void free_body_buffers(Buffers &b) {
   b.k0 = b.k1 = nullptr;
   b.v0 = b.v1 = b.hist = b.sys_of = nullptr;
   b.spos = nullptr;
-  b.bn_left = b.bn_right = b.bn_parent = b.bn_first = b.bn_last = b.bn_level = nullptr;
-  b.bn_flag = b.bin2cn = b.cn_bin = b.cn_child = b.cn_parent = nullptr;
+  b.bn_left = b.bn_right = b.bn_first = b.bn_last = b.bn_level = nullptr;
+  b.bn_rank = b.up_list = b.cn_bin = b.cn_child = b.cn_parent = nullptr;
   b.cn_meta = nullptr;
   b.cn_com = nullptr;
   b.cn_quad = b.cn_oct = nullptr;
@@ -183,15 +183,15 @@ int ensure_capacity(bh_system *s, int64_t n, int nsys, int n_items) {
     BH_CUDA(dalloc(&b.hist, b.hist_cap));
     BH_CUDA(dalloc(&b.sys_of, c));
     BH_CUDA(dalloc(&b.spos, c));
-    BH_CUDA(dalloc(&b.bn_left, c)); BH_CUDA(dalloc(&b.bn_right, c)); BH_CUDA(dalloc(&b.bn_parent, c));
+    BH_CUDA(dalloc(&b.bn_left, c)); BH_CUDA(dalloc(&b.bn_right, c));
     BH_CUDA(dalloc(&b.bn_first, c)); BH_CUDA(dalloc(&b.bn_last, c)); BH_CUDA(dalloc(&b.bn_level, c));
-    BH_CUDA(dalloc(&b.bn_flag, c)); BH_CUDA(dalloc(&b.bin2cn, c));
+    BH_CUDA(dalloc(&b.bn_rank, c)); BH_CUDA(dalloc(&b.up_list, c));
     BH_CUDA(dalloc(&b.cn_bin, c)); BH_CUDA(dalloc(&b.cn_meta, c)); BH_CUDA(dalloc(&b.cn_child, 8 * c));
     BH_CUDA(dalloc(&b.cn_parent, c)); BH_CUDA(dalloc(&b.cn_com, c));
     BH_CUDA(dalloc(&b.cn_quad, 6 * c)); BH_CUDA(dalloc(&b.cn_oct, 14 * c));
     BH_CUDA(dalloc(&b.cn_fq, 2 * c)); BH_CUDA(dalloc(&b.cn_fo, 4 * c));
     BH_CUDA(dalloc(&b.gflag, c + 1)); BH_CUDA(dalloc(&b.gscan, c + 1)); BH_CUDA(dalloc(&b.g_first, c + 1));
-    b.scan_tmp_cap = bh::scan_tmp_entries(c + 1);
+    b.scan_tmp_cap = bh::build_tmp_entries(c);
     BH_CUDA(dalloc(&b.scan_tmp, b.scan_tmp_cap));
     b.cap = c;
     b.nsys = 0;
@@ -248,6 +248,9 @@ int set_layout(bh_system *s, const int64_t *off, int nsys, cudaStream_t st) {
   BH_CUDA(cudaMemcpyAsync(b.items, items, (size_t)k * sizeof(bh::RedItem), cudaMemcpyHostToDevice, st));
   b.n_items = k;
   b.nsys = nsys;
+  b.sort_pairs = 0;
+  for (int q = 0; q < nsys; ++q)
+    b.sort_pairs += (double)(off[q + 1] - off[q]) * (double)(off[q + 1] - off[q]);
   bh::launch_layout(b, st);
   if (items == s->items_pin) {
     if (!s->layout_ev) BH_CUDA(cudaEventCreateWithFlags(&s->layout_ev, cudaEventDisableTiming));
@@ -314,14 +317,11 @@ void enqueue_build(bh_system *s, int keys_from_scalars, cudaStream_t st) {
   const int64_t n = s->n;
   const int L = p.depth;
   if (keys_from_scalars)
-    bh::launch_keys_only(s->x, s->y, s->z, n, L, b, st);
+    bh::launch_keys_only(s->m, s->x, s->y, s->z, n, L, b, st);
   else
     bh::launch_keys(s->m, s->x, s->y, s->z, n, L, p.amp, p.com_mode, b, st);
-  const int bits = (L == 0) ? 3 * bh::kMaxDepth : 3 * L;
-  bh::radix_sort_pairs(b.k0, b.v0, b.k1, b.v1, n, nullptr, bits, b.hist, &b.sc->err, st);
-  bh::launch_sort_by_system(n, b, st);
+  bh::launch_sort(s->m, s->x, s->y, s->z, n, L, b, st);
   if (L == 0) bh::launch_auto_depth(n, b, st);
-  bh::launch_gather(s->m, s->x, s->y, s->z, n, b, st);
   bh::launch_build_tree(n, L, b, st);
   bh::launch_upward(n, L, p.order, b, st);
   bh::launch_groups(n, p.group_size, p.group_span > 0 ? p.group_span : 2 * p.group_size, b, st);

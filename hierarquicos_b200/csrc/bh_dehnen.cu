@@ -44,6 +44,7 @@
 //     translated straight to it (down_bodies_kernel) instead of pushing level
 //     by level.  A body's force is m times its field.
 #include "bh_internal.cuh"
+#include "bh_lookback.cuh"
 
 namespace bh {
 
@@ -163,20 +164,6 @@ constexpr int kGenMutBits = 11;  // packed block scan: mutual count in the low b
 constexpr int kGenMutMask = (1 << kGenMutBits) - 1;
 static_assert(kGenTile < (1 << kGenMutBits), "a tile's mutual pairs fit the low bits");
 static_assert((int64_t)kGenTile * 36 << kGenMutBits < (1ll << 31), "the packed count fits an int");
-// tile words of the chained scan: top 2 bits the state, low 62 bits the count
-constexpr uint64_t kGenAggregate = 1ull << 62;  // the tile's own count
-constexpr uint64_t kGenInclusive = 2ull << 62;  // sum of the counts of tiles 0..t
-constexpr uint64_t kGenValue = (1ull << 62) - 1;
-constexpr int64_t kGenSpins = 1 << 22;          // polls of one look-back; about a second at most
-
-__device__ __forceinline__ uint64_t gen_ld(const uint64_t *p) {
-  uint64_t v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void gen_st(uint64_t *p, uint64_t v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 
 // Exclusive scan of one value per thread over the block; `ws` holds
 // kGenWarps ints; ends with a barrier so `ws` may be reused.
@@ -200,50 +187,6 @@ __device__ __forceinline__ int gen_block_scan(int v, int *ws, int *total) {
   *total = all;
   __syncthreads();
   return before + x - v;
-}
-
-// Prefix of the counts of the tiles before tile t in one status list, by one
-// whole warp: publish the tile's own count, then read the words of the 32
-// tiles before a window's end at once and add them up to the nearest
-// inclusive word (tile -1 counts as inclusive 0); a window with a word not yet
-// published is read again.  Only tiles claimed earlier -- by blocks that are
-// running and publish before they wait -- are waited for, and every wait is
-// bounded: a wait that gives up raises kErrTimeout.
-__device__ __forceinline__ int64_t gen_lookback(uint64_t *status, int t, int64_t count,
-                                                int *err) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  uint64_t *word = status + t;
-  if (t == 0) {
-    if (lane == 0) gen_st(word, kGenInclusive | (uint64_t)count);
-    return 0;
-  }
-  if (lane == 0) gen_st(word, kGenAggregate | (uint64_t)count);
-  int64_t excl = 0;
-  int j = t - 1;  // the window is tiles j - 31 .. j, lane k reading tile j - k
-  int64_t spins = 0;
-  for (;;) {
-    const int idx = j - lane;
-    const uint64_t w = idx >= 0 ? gen_ld(status + idx) : kGenInclusive;
-    const unsigned incl = __ballot_sync(0xffffffffu, (w & ~kGenValue) == kGenInclusive);
-    const unsigned unset = __ballot_sync(0xffffffffu, (w & ~kGenValue) == 0);
-    const int stop = incl ? __ffs(incl) - 1 : kWarp - 1;  // the last lane that counts
-    const unsigned counted = stop == kWarp - 1 ? 0xffffffffu : ((2u << stop) - 1u);
-    if (unset & counted) {
-      if (++spins > kGenSpins) {
-        if (lane == 0) atomicOr(err, kErrTimeout);
-        break;
-      }
-      continue;
-    }
-    int64_t v = lane <= stop ? (int64_t)(w & kGenValue) : 0;
-#pragma unroll
-    for (int o = kWarp / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    excl += v;
-    if (incl) break;
-    j -= kWarp;
-  }
-  if (lane == 0) gen_st(word, kGenInclusive | (uint64_t)(excl + count));
-  return excl;
 }
 
 // Classification of one input pair (a, b): kind 0 nothing, 1 the children
@@ -358,13 +301,13 @@ dual_gen_kernel(Ent e, const int2 *__restrict__ fin, const unsigned long long *_
     // the two chained scans, one warp each, at the same time
     const int warp = threadIdx.x / kWarp;
     if (warp == 0) {
-      const int64_t ef = gen_lookback(status_f, t, tot_f, err);
+      const int64_t ef = warp_lookback(status_f, t, tot_f, err);
       if (threadIdx.x == 0) {
         s_base[0] = ef;
         if ((int64_t)t == ntiles - 1) *nout = (unsigned long long)(ef + tot_f);
       }
     } else if (warp == 1) {
-      const int64_t em = gen_lookback(status_m, t, tot_m, err);
+      const int64_t em = warp_lookback(status_m, t, tot_m, err);
       if (threadIdx.x == kWarp) {
         s_base[1] = mut_base + em;
         if ((int64_t)t == ntiles - 1) *nmut_out = (unsigned long long)(mut_base + em + tot_m);
@@ -756,7 +699,7 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
   const int64_t nh = 2 * np;
   if (grow(d.keys, d.keys_cap, 2 * (nh > 0 ? nh : 1)) != cudaSuccess) return 1;
   if (grow(d.vals, d.vals_cap, 2 * (nh > 0 ? nh : 1)) != cudaSuccess) return 1;
-  if (grow(d.hist, d.hist_cap, radix_hist_entries(nh > 0 ? nh : 1)) != cudaSuccess) return 1;
+  if (grow(d.hist, d.hist_cap, radix_hist_entries(nh > 0 ? nh : 1, 4)) != cudaSuccess) return 1;
   cudaMemsetAsync(d.cnt, 0, (ne + 1) * sizeof(int32_t), s);
   const int32_t *sources = d.vals;  // the terms' sources in target order
   if (np > 0) {

@@ -72,6 +72,7 @@ struct Buffers {
   int sys_cap = 0;
   // batch layout
   int nsys = 0;
+  double sort_pairs = 0;           // sum of n_s^2 over the systems
   SysScalars *ss = nullptr;        // nsys entries
   SysScalars *ss_host = nullptr;   // host mirror
   int32_t *sys_of = nullptr;       // system of each body (same in input and key order)
@@ -90,11 +91,12 @@ struct Buffers {
   // sorted particles (x, y, z, m)
   double4 *spos = nullptr;
   // binary radix tree over the sorted keys (n - 1 internal nodes)
-  int32_t *bn_left = nullptr, *bn_right = nullptr, *bn_parent = nullptr;
+  int32_t *bn_left = nullptr, *bn_right = nullptr;
   int32_t *bn_first = nullptr, *bn_last = nullptr, *bn_level = nullptr;
-  int32_t *bn_flag = nullptr, *bin2cn = nullptr;
+  int32_t *bn_rank = nullptr;   // octree node's rank in its level, -1 none
+  int32_t *up_list = nullptr;   // upward pass: nodes that span its chunks
   // compact octree, ordered by (level, first particle)
-  int32_t *cn_bin = nullptr;
+  int32_t *cn_bin = nullptr;    // binary node of each octree node
   int4 *cn_meta = nullptr;       // first, count, level, nchild
   int32_t *cn_child = nullptr;   // 8 per node; >= 0 node, < 0 particle ~p
   int32_t *cn_parent = nullptr;
@@ -133,8 +135,8 @@ void launch_verify_keys(const double *x, const double *y, const double *z, int64
                         Buffers &b, cudaStream_t s);
 void launch_auto_depth(int64_t n, Buffers &b, cudaStream_t s);
 void launch_adopt_seq_com(Buffers &b, cudaStream_t s);
-void launch_keys_only(const double *x, const double *y, const double *z, int64_t n, int L,
-                      Buffers &b, cudaStream_t s);
+void launch_keys_only(const double *m, const double *x, const double *y, const double *z, int64_t n,
+                      int L, Buffers &b, cudaStream_t s);
 void set_seq_com_smem_limit();
 inline int grid_for(int64_t n, int threads, int cap) {
   int64_t g = (n + threads - 1) / threads;
@@ -159,15 +161,26 @@ cudaError_t hostcopy_upload(HostCopy *h, const double *const *src, double *const
 cudaError_t hostcopy_download(HostCopy *h, double *dst, const double *src, int64_t n,
                               cudaStream_t st);
 
-// stable LSD radix sort of (key, value) pairs over bits [0, bits); the
-// result ends in (k0, v0).  n_dev, when given, holds the element count on the
-// device (n is then an upper bound).  A look-back wait that gives up sets
-// kErrTimeout in *err (device).
-void radix_sort_pairs(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                      const int32_t *n_dev, int bits, int32_t *hist, int *err, cudaStream_t s);
-// the same for 32-bit keys when only the values are wanted: the last pass
-// writes no keys and nothing is copied back; returns the buffer holding the
-// sorted values (0: v0, 1: v1).  key_counts, if given, holds the number of keys
+// How the bodies of a batch are brought into (system, key) order: by counting
+// ranks (keys start in k1), or by a stable LSD radix sort of kpass key digits and
+// spass digits of the system, whose passes end in k0 and v0; scratch int32
+// entries of b.hist are cleared before.
+constexpr int kMaxSortPasses = 11;  // 8 of the key, 3 of the system (at most 2^24 systems)
+struct SortPlan {
+  bool by_rank;
+  int kpass, spass;
+  int64_t scratch;
+};
+SortPlan sort_plan(int64_t n, int L, const Buffers &b);
+// Sorted keys (k0), permutation (v0) and bodies (spos) from the keys that
+// launch_keys / launch_keys_only left.  A look-back wait that gives up sets
+// kErrTimeout.
+void launch_sort(const double *m, const double *x, const double *y, const double *z, int64_t n,
+                 int L, Buffers &b, cudaStream_t s);
+
+// stable LSD radix sort of 32-bit keys over bits [0, bits) when only the values
+// are wanted: the last pass writes no keys and nothing is copied back; returns
+// the buffer holding the sorted values (0: v0, 1: v1).  key_counts, if given, holds the number of keys
 // of every key value 0..n_key_values-1 (the digit counts then come from it
 // instead of from a pass over the keys).
 int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n, int bits,
@@ -177,21 +190,29 @@ int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, in
 // 8192-value tile; scratch of the radix sort: digit counts of 8 passes x 256
 // digits, 8 tile counters, and a 64-bit word per (pass, 4096-key tile, digit)
 constexpr int64_t scan_tmp_entries(int64_t n) { return 2 * ((n + 8191) / 8192) + 4; }
+// scratch of the tree, group and upward passes of a build (layout: bh_tree.cu),
+// in int32 entries
+constexpr int64_t kTreeTile = 256, kGroupScanTile = 2048;
+constexpr int64_t upward_counter_entries(int64_t n) { return (n >> 15) + (n >> 22) + (n >> 29) + 4; }
+constexpr int64_t build_tmp_entries(int64_t n) {
+  return 2 + kWarp + 2 * kWarp * ((n + kTreeTile - 1) / kTreeTile) +
+         2 * ((n + kGroupScanTile - 1) / kGroupScanTile) + upward_counter_entries(n);
+}
 // radix sort tiles: sorts of at most kSortSmallMax keys use small tiles (more
 // blocks in flight: a 2^14-body build 0.380 -> 0.350 ms), larger ones large
 // tiles (fewer look-back words and less scratch to clear: with small tiles
 // the 2^20-body build took 0.873 instead of 0.821 ms)
 constexpr int64_t kSortTileLarge = 4096, kSortTileSmall = 1024, kSortSmallMax = (int64_t)1 << 16;
 constexpr int64_t sort_tile(int64_t n) { return n <= kSortSmallMax ? kSortTileSmall : kSortTileLarge; }
-constexpr int64_t radix_hist_entries(int64_t n) {
-  // the most tiles any sort of up to n keys uses
-  return 8 * 256 + 8 +
-         2 * 8 * 256 *
-             ((((n < kSortSmallMax ? n : kSortSmallMax) + kSortTileSmall - 1) / kSortTileSmall >
-                       (n + kSortTileLarge - 1) / kSortTileLarge
-                   ? ((n < kSortSmallMax ? n : kSortSmallMax) + kSortTileSmall - 1) / kSortTileSmall
-                   : (n + kSortTileLarge - 1) / kSortTileLarge) +
-              1);
+// 32-bit words of the digit counts and tile counters, then 64-bit tile words of
+// `passes` passes over n keys (the most of any sort of up to n keys)
+constexpr int64_t radix_tiles(int64_t n) {
+  const int64_t small = ((n < kSortSmallMax ? n : kSortSmallMax) + kSortTileSmall - 1) / kSortTileSmall;
+  const int64_t large = (n + kSortTileLarge - 1) / kSortTileLarge;
+  return (small > large ? small : large) + 1;
+}
+constexpr int64_t radix_hist_entries(int64_t n, int passes = kMaxSortPasses) {
+  return passes * 256 + 12 + 2 * passes * 256 * radix_tiles(n);
 }
 
 // exclusive scan of n int32 values in one launch; total written to *total
@@ -201,12 +222,9 @@ void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n
                     int32_t *total, int32_t *tmp, int *err, cudaStream_t s,
                     int32_t *total2 = nullptr);
 
-void launch_gather(const double *m, const double *x, const double *y, const double *z, int64_t n,
-                   Buffers &b, cudaStream_t s);
-// after the key sort of a batch: stable sort by system, so that every system's
-// bodies are again contiguous, in key order
-void launch_sort_by_system(int64_t n, Buffers &b, cudaStream_t s);
 void launch_build_tree(int64_t n, int L, Buffers &b, cudaStream_t s);
+// the upward pass's list counters (cleared by launch_build_tree)
+int32_t *upward_counters(int64_t n, Buffers &b);
 void launch_upward(int64_t n, int L, int order, Buffers &b, cudaStream_t s);
 void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaStream_t s);
 

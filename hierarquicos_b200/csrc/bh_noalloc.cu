@@ -48,7 +48,7 @@ constexpr int64_t kStackCap = kMaxN;  // stack entries per warp: a group's walk 
                                       // node at most once and a tree of n bodies has fewer
                                       // than n nodes, so the stack cannot overflow
 constexpr int64_t kItems = (kMaxN + bh::kRedChunk - 1) / bh::kRedChunk;  // reduction items
-constexpr int kNumBufs = 36;
+constexpr int kNumBufs = 35;
 
 constexpr int64_t align256(int64_t x) { return (x + 255) & ~int64_t(255); }
 
@@ -69,7 +69,7 @@ constexpr Sizes buffer_bytes(int64_t c) {
   z.v[i++] = 4 * c;                                   // sys_of
   z.v[i++] = (int64_t)sizeof(bh::RedItem) * kItems;    // items
   z.v[i++] = 32 * c;                                  // spos
-  for (int k = 0; k < 8; ++k) z.v[i++] = 4 * c;       // bn_* and bin2cn
+  for (int k = 0; k < 7; ++k) z.v[i++] = 4 * c;       // bn_* and up_list
   z.v[i++] = 4 * c;                                   // cn_bin
   z.v[i++] = 16 * c;                                  // cn_meta
   z.v[i++] = 32 * c;                                  // cn_child
@@ -83,7 +83,7 @@ constexpr Sizes buffer_bytes(int64_t c) {
   z.v[i++] = 4 * (c + 1);                             // gflag
   z.v[i++] = 4 * (c + 1);                             // gscan
   z.v[i++] = 4 * (c + 1);                             // g_first
-  z.v[i++] = 4 * bh::scan_tmp_entries(c + 1);         // scan_tmp
+  z.v[i++] = 4 * bh::build_tmp_entries(c);            // scan_tmp
   z.v[i++] = 4 * kSlots * kStackCap;                  // wstack
   z.v[i++] = 32;                                      // counters
   z.v[i++] = 32;                                      // stats
@@ -114,8 +114,8 @@ bh::Buffers carve(unsigned char *base) {
   bh::Buffers b;
   take(b.k0); take(b.k1); take(b.v0); take(b.v1); take(b.hist); take(b.partials); take(b.ss);
   take(b.sys_of); take(b.items); take(b.spos);
-  take(b.bn_left); take(b.bn_right); take(b.bn_parent); take(b.bn_first); take(b.bn_last);
-  take(b.bn_level); take(b.bn_flag); take(b.bin2cn);
+  take(b.bn_left); take(b.bn_right); take(b.bn_first); take(b.bn_last);
+  take(b.bn_level); take(b.bn_rank); take(b.up_list);
   take(b.cn_bin); take(b.cn_meta); take(b.cn_child); take(b.cn_parent); take(b.cn_com);
   take(b.cn_quad); take(b.cn_oct); take(b.cn_fq); take(b.cn_fo); take(b.level_begin);
   take(b.gflag); take(b.gscan); take(b.g_first); take(b.scan_tmp); take(b.wstack);
@@ -124,7 +124,7 @@ bh::Buffers carve(unsigned char *base) {
   b.sys_cap = 1;
   b.items_cap = (int)kItems;
   b.hist_cap = bh::radix_hist_entries(kMaxN);
-  b.scan_tmp_cap = bh::scan_tmp_entries(kMaxN + 1);
+  b.scan_tmp_cap = bh::build_tmp_entries(kMaxN);
   b.wstack_cap = kStackCap;
   b.wstack_slots = kSlots;
   return b;

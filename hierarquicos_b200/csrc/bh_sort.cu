@@ -19,6 +19,7 @@
 // claimed before its own, by blocks that are already running; every wait is
 // bounded and a wait that gives up raises an error flag instead of hanging.
 #include "bh_internal.cuh"
+#include "bh_lookback.cuh"
 
 namespace bh {
 
@@ -30,7 +31,13 @@ constexpr int kItems = 16;       // keys per thread of a large sort's tile
 constexpr int kSmallItems = kSortTileSmall / 256;  // and of a small sort's
 constexpr int kTile = kSortThreads * kItems;  // 4096 keys per block (large sorts)
 constexpr int kRadix = 256;
-constexpr int kMaxPasses = 8;  // 64-bit keys
+
+// Sum over the systems of n_s^2 up to which a batch is sorted by counting; above
+// it the comparisons cost more than the radix passes.  Whole builds, us, counting
+// / radix: one system of 1,024 bodies 80 / 125, 8,192 109 / 156, 16,384 156 / 161,
+// 20,000 213 / 164; batches (whose radix sort has passes over the system too) of
+// 1.4e8 218 / 298, 6.7e8 352 / 322, 1.5e9 535 / 338.
+constexpr double kRankPairsOne = 2.8e8, kRankPairsBatch = 4e8;
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
@@ -72,43 +79,13 @@ __device__ int block_excl_scan(int v, int *ws, int *total) {
   return off + incl - v;
 }
 
-// Digit histograms of all passes: ghist[p][d] = number of keys whose digit p
-// is d (warp-aggregated shared-memory counts, then one global add per bin).
-template <typename K>
-__global__ void __launch_bounds__(kSortThreads)
-digit_hist_kernel(const K *__restrict__ keys, int64_t n_max, const int32_t *n_dev,
-                  int passes, uint32_t *__restrict__ ghist) {
-  __shared__ uint32_t h[kMaxPasses][kRadix];
-  const int lane = threadIdx.x & (kWarp - 1);
-  const int64_t n = n_dev ? bh_min64(n_max, (int64_t)*n_dev) : n_max;
-  for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kSortThreads) (&h[0][0])[i] = 0;
-  __syncthreads();
-  const unsigned lt = lanemask_lt();
-  const int64_t stride = (int64_t)gridDim.x * kSortThreads;
-  for (int64_t base = (int64_t)blockIdx.x * kSortThreads; base < n; base += stride) {
-    const int64_t idx = base + threadIdx.x;
-    const bool valid = idx < n;
-    const K k = valid ? keys[idx] : (K)0;
-    for (int p = 0; p < passes; ++p) {
-      const int d = valid ? (int)((k >> (8 * p)) & 0xff) : kRadix;
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
-      if (d < kRadix && (peers & lt) == 0) atomicAdd(&h[p][d], (uint32_t)__popc(peers));
-    }
-    (void)lane;
-  }
-  __syncthreads();
-  for (int p = 0; p < passes; ++p) {
-    const uint32_t c = h[p][threadIdx.x];  // kSortThreads == kRadix
-    if (c) atomicAdd(&ghist[p * kRadix + threadIdx.x], c);
-  }
-}
-
-// The same digit counts from the number of keys of every key value v (keys are
-// the values 0..n_values-1): pass p's count of digit d sums count[v] over the
+// Digit counts from the number of keys of every key value v (keys are the
+// values 0..n_values-1): pass p's count of digit d sums count[v] over the
 // values whose digit p is d -- one read of the counts instead of all keys.
 __global__ void __launch_bounds__(kSortThreads)
 count_hist_kernel(const int32_t *__restrict__ count, int64_t n_values, int passes,
                   uint32_t *__restrict__ ghist) {
+  constexpr int kMaxPasses = 4;  // 32-bit keys
   __shared__ uint32_t h[kMaxPasses][kRadix];
   for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kSortThreads) (&h[0][0])[i] = 0;
   __syncthreads();
@@ -125,35 +102,11 @@ count_hist_kernel(const int32_t *__restrict__ count, int64_t n_values, int passe
   }
 }
 
-// Exclusive scan of each pass's 256 digit counts, in place.
-__global__ void __launch_bounds__(kSortThreads) digit_scan_kernel(uint32_t *ghist, int passes) {
-  __shared__ int ws[kSortWarps];
-  for (int p = 0; p < passes; ++p) {
-    const int v = (int)ghist[p * kRadix + threadIdx.x];
-    const int ex = block_excl_scan(v, ws, nullptr);
-    ghist[p * kRadix + threadIdx.x] = (uint32_t)ex;
-  }
-}
-
-// tile words: top 2 bits the state, low 62 bits the count
-constexpr uint64_t kTileAggregate = 1ull << 62;  // the tile's own count
-constexpr uint64_t kTileInclusive = 2ull << 62;  // sum of the counts of tiles 0..t
-constexpr uint64_t kTileValue = (1ull << 62) - 1;
-constexpr int64_t kLookbackSpins = 1 << 22;     // per word; about a second at most
-
-__device__ __forceinline__ uint64_t ld_relaxed(const uint64_t *p) {
-  uint64_t v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(uint64_t *p, uint64_t v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-template <typename K, int ITEMS>
+template <typename K, int ITEMS, bool SYS>
 struct PassSmem {
   K sk[ITEMS * kSortThreads];
   int32_t sv[ITEMS * kSortThreads];
+  unsigned char sd[SYS ? ITEMS * kSortThreads : 16];  // digits that the key does not hold
   int wh[kSortWarps][kRadix];
   int tile_start[kRadix];
   int gbase[kRadix];
@@ -165,14 +118,17 @@ struct PassSmem {
 // keys nobody reads).
 // 3 blocks per SM (80 registers, no spills; the compiler's own choice was 128
 // and 2 blocks): the 181 M-term sort of Dehnen's method 1 ms faster.
-template <typename K, int ITEMS>
+// counts: the pass's 256 digit counts, which every block scans itself.  sys_of
+// given: the digit is the system's (of the body that the value names), not the
+// key's.
+template <typename K, int ITEMS, bool SYS>
 __global__ void __launch_bounds__(kSortThreads, 3)
 onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
-                K *__restrict__ kout, int32_t *__restrict__ vout, int64_t n_max,
-                const int32_t *n_dev, int shift, const uint32_t *__restrict__ gofs,
+                K *__restrict__ kout, int32_t *__restrict__ vout, int64_t n, int shift,
+                const int32_t *__restrict__ sys_of, const uint32_t *__restrict__ counts,
                 uint64_t *__restrict__ tiles, int32_t *__restrict__ tile_ctr, int *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  PassSmem<K, ITEMS> &S = *reinterpret_cast<PassSmem<K, ITEMS> *>(smem_raw);
+  PassSmem<K, ITEMS, SYS> &S = *reinterpret_cast<PassSmem<K, ITEMS, SYS> *>(smem_raw);
   constexpr int kItems = ITEMS;
   constexpr int kTile = ITEMS * kSortThreads;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
@@ -180,7 +136,6 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
   for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) (&S.wh[0][0])[i] = 0;
   __syncthreads();
   const int t = S.tile;
-  const int64_t n = n_dev ? bh_min64(n_max, (int64_t)*n_dev) : n_max;
   const int64_t tile_base = (int64_t)t * kTile;
   if (tile_base >= n) return;  // uniform across the block; later tiles return too
   const int tile_n = (int)bh_min64(kTile, n - tile_base);
@@ -195,7 +150,7 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
     bool valid = li < tile_n;
     k[i] = valid ? kin[tile_base + li] : (K)0;
     v[i] = valid ? vin[tile_base + li] : 0;
-    dig[i] = valid ? (int)((k[i] >> shift) & 0xff) : kRadix;
+    dig[i] = valid ? (int)(((SYS ? (K)sys_of[v[i]] : k[i]) >> shift) & 0xff) : kRadix;
   }
   const unsigned lt = lanemask_lt();
 #pragma unroll
@@ -220,27 +175,8 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
     cnt += c;
   }
   // publish, then look back over the earlier tiles for this digit
-  uint64_t *word = tiles + (int64_t)t * kRadix + d;
-  int64_t excl = 0;
-  if (t == 0) {
-    st_relaxed(word, kTileInclusive | (uint64_t)cnt);
-  } else {
-    st_relaxed(word, kTileAggregate | (uint64_t)cnt);
-    int j = t - 1;
-    int64_t spins = 0;
-    while (j >= 0) {
-      const uint64_t w = ld_relaxed(tiles + (int64_t)j * kRadix + d);
-      if ((w & ~kTileValue) == 0) {
-        if (++spins > kLookbackSpins) { atomicOr(err, kErrTimeout); break; }
-        continue;
-      }
-      excl += (int64_t)(w & kTileValue);
-      if ((w & ~kTileValue) == kTileInclusive) break;
-      --j;
-    }
-    st_relaxed(word, kTileInclusive | (uint64_t)(excl + cnt));
-  }
-  S.gbase[d] = (int)(gofs[d] + excl);
+  const int64_t excl = thread_lookback(tiles + d, t, kRadix, cnt, err);
+  S.gbase[d] = block_excl_scan((int)counts[d], S.ws, nullptr) + (int)excl;
   int start = block_excl_scan(cnt, S.ws, nullptr);
   S.tile_start[d] = start;
   __syncthreads();
@@ -251,12 +187,13 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
       int pos = S.tile_start[dd] + S.wh[warp][dd] + rank[i];
       S.sk[pos] = k[i];
       S.sv[pos] = v[i];
+      if (SYS) S.sd[pos] = (unsigned char)dd;
     }
   }
   __syncthreads();
   for (int j = threadIdx.x; j < tile_n; j += kSortThreads) {
     const K key = S.sk[j];
-    const int dd = (int)((key >> shift) & 0xff);
+    const int dd = SYS ? (int)S.sd[j] : (int)((key >> shift) & 0xff);
     const int64_t o = (int64_t)S.gbase[dd] + (j - S.tile_start[dd]);
     if (kout) kout[o] = key;
     vout[o] = S.sv[j];
@@ -296,30 +233,14 @@ scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, i
   }
   int tile_total;
   int off = block_excl_scan(sum, ws, &tile_total);
-  if (threadIdx.x == 0) {
-    int64_t excl = 0;
-    if (t == 0) {
-      st_relaxed(words, kTileInclusive | (uint64_t)tile_total);
-    } else {
-      st_relaxed(words + t, kTileAggregate | (uint64_t)tile_total);
-      int j = t - 1;
-      int64_t spins = 0;
-      while (j >= 0) {
-        const uint64_t w = ld_relaxed(words + j);
-        if ((w & ~kTileValue) == 0) {
-          if (++spins > kLookbackSpins) { atomicOr(err, kErrTimeout); break; }
-          continue;
-        }
-        excl += (int64_t)(w & kTileValue);
-        if ((w & ~kTileValue) == kTileInclusive) break;
-        --j;
+  if (threadIdx.x < kWarp) {
+    const int64_t excl = warp_lookback(words, t, tile_total, err);
+    if (threadIdx.x == 0) {
+      s_excl = excl;
+      if ((int64_t)t == ntiles - 1) {
+        if (total_out) *total_out = (int32_t)(excl + tile_total);
+        if (total_out2) *total_out2 = (int32_t)(excl + tile_total);
       }
-      st_relaxed(words + t, kTileInclusive | (uint64_t)(excl + tile_total));
-    }
-    s_excl = excl;
-    if ((int64_t)t == ntiles - 1) {
-      if (total_out) *total_out = (int32_t)(excl + tile_total);
-      if (total_out2) *total_out2 = (int32_t)(excl + tile_total);
     }
   }
   __syncthreads();
@@ -331,64 +252,156 @@ scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, i
   }
 }
 
+// bodies into key order, from the packed copy the keys kernel wrote
 __global__ void __launch_bounds__(256)
-gather_kernel(const double *__restrict__ m, const double *__restrict__ x,
-              const double *__restrict__ y, const double *__restrict__ z,
-              const int32_t *__restrict__ perm, int64_t n, double4 *__restrict__ spos) {
+gather_kernel(const double4 *__restrict__ packed, const int32_t *__restrict__ perm, int64_t n,
+              double4 *__restrict__ spos) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t p = perm[i];
-    spos[i] = make_double4(x[p], y[p], z[p], m[p]);
+       i += (int64_t)gridDim.x * blockDim.x)
+    spos[i] = packed[perm[i]];
+}
+
+// ---- sort by counting (small systems) ----
+
+// Body t's place in its system's key order is the number of that system's keys
+// below its own, equal keys of earlier bodies included (the stable order): with
+// few bodies counting all of them beats eight dependent passes.  A block takes
+// 64 bodies, two per lane, and its 8 warps a slice of the system's keys each (two
+// keys per shared-memory read, three instructions a comparison); the bodies then
+// go straight to their places, so there is no gather either.
+// Bound: the integer pipe, n_s^2 comparisons (1,024 bodies 6 us against 45 for
+// eight radix passes and their counts; kRankPairsOne has the crossing).
+constexpr int kRankWarps = 8, kRankBodies = 2 * kWarp;
+
+// neg -= (a < b), on the borrow of a - b
+__device__ __forceinline__ void count_below(unsigned &neg, uint64_t a, uint64_t b) {
+  asm("{\n\t.reg .u32 t, al, ah, bl, bh;\n\t"
+      "mov.b64 {al, ah}, %1;\n\tmov.b64 {bl, bh}, %2;\n\t"
+      "sub.cc.u32 t, al, bl;\n\tsubc.cc.u32 t, ah, bh;\n\tsubc.u32 %0, %0, 0;\n\t}"
+      : "+r"(neg) : "l"(a), "l"(b));
+}
+
+__global__ void __launch_bounds__(kRankWarps *kWarp)
+rank_sort_kernel(const uint64_t *__restrict__ keys, const double *__restrict__ m,
+                 const double *__restrict__ x, const double *__restrict__ y,
+                 const double *__restrict__ z, int64_t n, const int32_t *__restrict__ sys_of,
+                 const SysScalars *__restrict__ sys, uint64_t *__restrict__ kout,
+                 int32_t *__restrict__ vout, double4 *__restrict__ spos) {
+  __shared__ __align__(16) uint64_t tile[kRankWarps][2 * kWarp];
+  __shared__ unsigned part[kRankWarps][kRankBodies];
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  const int64_t base = (int64_t)blockIdx.x * kRankBodies;
+  int64_t t[2];
+  uint64_t key[2];
+  int mine[2];
+  unsigned neg[2] = {0, 0};
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    t[q] = base + q * kWarp + lane;
+    key[q] = t[q] < n ? keys[t[q]] : 0;
+    mine[q] = t[q] < n ? sys_of[t[q]] : -1;
+  }
+  const int s_last = sys_of[bh_min64(base + kRankBodies, n) - 1];
+  for (int s = sys_of[base]; s <= s_last; ++s) {
+    const int64_t off = sys[s].off, ns = sys[s].n;
+    const int64_t b = off + ns * (warp + 1) / kRankWarps;
+    for (int64_t a = off + ns * warp / kRankWarps; a < b; a += 2 * kWarp) {
+      // keys beyond the slice never count
+      tile[warp][lane] = a + lane < b ? keys[a + lane] : ~0ull;
+      tile[warp][kWarp + lane] = a + kWarp + lane < b ? keys[a + kWarp + lane] : ~0ull;
+      __syncwarp();
+      const ulonglong2 *k2 = reinterpret_cast<const ulonglong2 *>(tile[warp]);
+      if (a + 2 * kWarp <= base || a >= base + kRankBodies) {
+        // all earlier bodies (equal keys count: below key + 1) or all later ones
+        const uint64_t up = a < base ? 1 : 0;
+        const uint64_t b0 = mine[0] == s ? key[0] + up : 0, b1 = mine[1] == s ? key[1] + up : 0;
+#pragma unroll 8
+        for (int j = 0; j < kWarp; ++j) {
+          const ulonglong2 k = k2[j];
+          count_below(neg[0], k.x, b0); count_below(neg[0], k.y, b0);
+          count_below(neg[1], k.x, b1); count_below(neg[1], k.y, b1);
+        }
+      } else {
+        for (int j = 0; j < kWarp; ++j) {
+          const ulonglong2 k = k2[j];
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (mine[q] != s) continue;
+            count_below(neg[q], k.x, key[q] + (a + 2 * j < t[q] ? 1 : 0));
+            count_below(neg[q], k.y, key[q] + (a + 2 * j + 1 < t[q] ? 1 : 0));
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) part[warp][q * kWarp + lane] = neg[q];
+  __syncthreads();
+  if (threadIdx.x < kRankBodies && base + threadIdx.x < n) {
+    unsigned c = 0;
+#pragma unroll
+    for (int w = 0; w < kRankWarps; ++w) c -= part[w][threadIdx.x];
+    const int64_t p = base + threadIdx.x, o = sys[sys_of[p]].off + c;
+    kout[o] = keys[p];
+    vout[o] = (int32_t)p;
+    spos[o] = make_double4(x[p], y[p], z[p], m[p]);
   }
 }
 
-// stage 2 of a batch sort: key = system of the body at sorted position i
-__global__ void __launch_bounds__(256)
-sys_keys_kernel(const int32_t *__restrict__ perm, const int32_t *__restrict__ sys_of, int64_t n,
-                uint64_t *__restrict__ ck, int32_t *__restrict__ cv) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    ck[i] = (uint64_t)sys_of[perm[i]];
-    cv[i] = (int32_t)i;
-  }
-}
-
-__global__ void __launch_bounds__(256)
-regather_kernel(const uint64_t *__restrict__ k0, const int32_t *__restrict__ v0,
-                const int32_t *__restrict__ order, int64_t n, uint64_t *__restrict__ k1,
-                int32_t *__restrict__ v1) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t j = order[i];
-    k1[i] = k0[j];
-    v1[i] = v0[j];
-  }
-}
-
-template <typename K, int ITEMS>
-void set_pass_smem() {
-  static bool done = false;  // a function attribute: once per process
-  if (!done) {
-    cudaFuncSetAttribute(onesweep_kernel<K, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(PassSmem<K, ITEMS>));
-    done = true;
-  }
-}
-
-template <typename K, int ITEMS>
+template <typename K, int ITEMS, bool SYS>
 void launch_pass(int64_t ntiles, const K *ki, const int32_t *vi, K *ko, int32_t *vo, int64_t n,
-                 const int32_t *n_dev, int shift, const uint32_t *gofs, uint64_t *tiles,
+                 int shift, const int32_t *sys_of, const uint32_t *counts, uint64_t *tiles,
                  int32_t *ctr, int *err, cudaStream_t s) {
-  set_pass_smem<K, ITEMS>();
-  onesweep_kernel<K, ITEMS><<<(unsigned)(ntiles > 0 ? ntiles : 1), kSortThreads,
-                              sizeof(PassSmem<K, ITEMS>), s>>>(ki, vi, ko, vo, n, n_dev, shift,
-                                                               gofs, tiles, ctr, err);
+  constexpr int smem = (int)sizeof(PassSmem<K, ITEMS, SYS>);
+  static bool done[64] = {};  // the limit is set once per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (!done[dev]) {
+    cudaFuncSetAttribute(onesweep_kernel<K, ITEMS, SYS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         smem);
+    done[dev] = true;
+  }
+  onesweep_kernel<K, ITEMS, SYS><<<(unsigned)ntiles, kSortThreads, smem, s>>>(
+      ki, vi, ko, vo, n, shift, sys_of, counts, tiles, ctr, err);
+}
+
+// scratch layout (int32 entries): digit counts [passes][256], tile counters
+// [12], then the tile words (uint64) [passes][ntiles][256]
+struct SortScratch {
+  uint32_t *counts;
+  int32_t *ctr;
+  uint64_t *tiles;
+  int64_t ntiles, entries;
+};
+SortScratch sort_scratch(int64_t n, int passes, int32_t *hist) {
+  SortScratch c;
+  c.counts = reinterpret_cast<uint32_t *>(hist);
+  c.ctr = hist + passes * kRadix;
+  c.tiles = reinterpret_cast<uint64_t *>(hist + passes * kRadix + 12);
+  c.ntiles = (n + sort_tile(n) - 1) / sort_tile(n);
+  c.entries = passes * kRadix + 12 + 2 * (int64_t)passes * c.ntiles * kRadix;
+  return c;
+}
+
+template <typename K, bool SYS>
+void one_pass(const SortScratch &c, int pass, int64_t n, int shift, const int32_t *sys_of, const K *ki,
+              const int32_t *vi, K *ko, int32_t *vo, int *err, cudaStream_t s) {
+  // small sorts take small tiles: more blocks in flight for the same keys
+  if (sort_tile(n) == kSortTileSmall)
+    launch_pass<K, kSmallItems, SYS>(c.ntiles, ki, vi, ko, vo, n, shift, sys_of,
+                                     c.counts + pass * kRadix, c.tiles + pass * c.ntiles * kRadix,
+                                     c.ctr + pass, err, s);
+  else
+    launch_pass<K, kItems, SYS>(c.ntiles, ki, vi, ko, vo, n, shift, sys_of, c.counts + pass * kRadix,
+                                c.tiles + pass * c.ntiles * kRadix, c.ctr + pass, err, s);
 }
 
 }  // namespace
 
-static_assert(kScanChunk == 8192 && kTile == kSortTileLarge && kRadix == 256 && kMaxPasses == 8 &&
-                  kSortThreads * kSmallItems == kSortTileSmall,
+static_assert(kScanChunk == 8192 && kTile == kSortTileLarge && kRadix == 256 &&
+                  kSortThreads * kSmallItems == kSortTileSmall && kMaxSortPasses <= 12,
               "scan_tmp_entries / radix_hist_entries in bh_internal.cuh assume these sizes");
 
 void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n_dev,
@@ -399,86 +412,61 @@ void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n
   scan_onepass_kernel<<<nb, kScanThreads, 0, s>>>(in, out, n, n_dev, tmp, total, total2, err);
 }
 
-// The passes of one sort; returns the buffer (0: k0/v0, 1: k1/v1) that holds
-// the result.  With keys_out false the last pass writes only the values.
-template <typename K>
-static int sort_passes(K *k0, int32_t *v0, K *k1, int32_t *v1, int64_t n, const int32_t *n_dev,
-                       int bits, int32_t *hist, int *err, bool keys_out, cudaStream_t s,
-                       const int32_t *key_counts = nullptr, int64_t n_key_values = 0) {
-  // small sorts take small tiles: more blocks in flight for the same keys
-  const int64_t tile = sort_tile(n);
-  const int64_t ntiles = (n + tile - 1) / tile;
+int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n, int bits,
+                        int32_t *hist, int *err, cudaStream_t s, const int32_t *key_counts,
+                        int64_t n_key_values) {
   int passes = (bits + 7) / 8;
-  if (passes < 1) passes = 1;
-  if (passes > (int)sizeof(K)) passes = (int)sizeof(K);
-  // scratch layout (int32 entries): digit counts [8][256], tile counters [8],
-  // then the tile words (uint64) [passes][ntiles][256]
-  uint32_t *ghist = reinterpret_cast<uint32_t *>(hist);
-  int32_t *ctr = hist + kMaxPasses * kRadix;
-  uint64_t *tiles = reinterpret_cast<uint64_t *>(hist + kMaxPasses * kRadix + kMaxPasses);
-  const int64_t used = kMaxPasses * kRadix + kMaxPasses + 2 * (int64_t)passes * ntiles * kRadix;
-  cudaMemsetAsync(hist, 0, used * sizeof(int32_t), s);
-  if (key_counts)
-    count_hist_kernel<<<grid_for(n_key_values, kSortThreads, 148 * 8), kSortThreads, 0, s>>>(
-        key_counts, n_key_values, passes, ghist);
-  else
-    digit_hist_kernel<K><<<grid_for(n, kSortThreads, 148 * 8), kSortThreads, 0, s>>>(k0, n, n_dev,
-                                                                                     passes, ghist);
-  digit_scan_kernel<<<1, kSortThreads, 0, s>>>(ghist, passes);
-  K *ki = k0, *ko = k1;
+  passes = passes < 1 ? 1 : (passes > 4 ? 4 : passes);
+  const SortScratch c = sort_scratch(n, passes, hist);
+  cudaMemsetAsync(hist, 0, c.entries * sizeof(int32_t), s);
+  count_hist_kernel<<<grid_for(n_key_values, kSortThreads, 148 * 8), kSortThreads, 0, s>>>(
+      key_counts, n_key_values, passes, c.counts);
+  uint32_t *ki = k0, *ko = k1;
   int32_t *vi = v0, *vo = v1;
   for (int p = 0; p < passes; ++p) {
-    K *kw = (p == passes - 1 && !keys_out) ? nullptr : ko;
-    if (tile == kSortTileSmall)
-      launch_pass<K, kSmallItems>(ntiles, ki, vi, kw, vo, n, n_dev, 8 * p, ghist + p * kRadix,
-                                  tiles + (int64_t)p * ntiles * kRadix, ctr + p, err, s);
-    else
-      launch_pass<K, kItems>(ntiles, ki, vi, kw, vo, n, n_dev, 8 * p, ghist + p * kRadix,
-                             tiles + (int64_t)p * ntiles * kRadix, ctr + p, err, s);
-    K *tk = ki; ki = ko; ko = tk;
+    one_pass<uint32_t, false>(c, p, n, 8 * p, nullptr, ki, vi, p == passes - 1 ? nullptr : ko, vo, err, s);
+    uint32_t *tk = ki; ki = ko; ko = tk;
     int32_t *tv = vi; vi = vo; vo = tv;
   }
   return ki == k0 ? 0 : 1;
 }
 
-void radix_sort_pairs(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                      const int32_t *n_dev, int bits, int32_t *hist, int *err, cudaStream_t s) {
-  if (sort_passes<uint64_t>(k0, v0, k1, v1, n, n_dev, bits, hist, err, true, s) == 1) {
-    // odd number of passes: the result sits in the second buffer
-    cudaMemcpyAsync(k0, k1, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(v0, v1, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
+SortPlan sort_plan(int64_t n, int L, const Buffers &b) {
+  SortPlan p;
+  p.by_rank = b.sort_pairs <= (b.nsys > 1 ? kRankPairsBatch : kRankPairsOne);
+  const int bits = 3 * (L == 0 ? kMaxDepth : L);
+  p.kpass = (bits + 7) / 8;
+  p.spass = 0;
+  while (((int64_t)1 << (8 * p.spass)) < b.nsys) ++p.spass;
+  p.scratch = sort_scratch(n, p.kpass + p.spass, nullptr).entries;
+  return p;
+}
+
+void launch_sort(const double *m, const double *x, const double *y, const double *z, int64_t n,
+                 int L, Buffers &b, cudaStream_t s) {
+  const SortPlan plan = sort_plan(n, L, b);
+  if (plan.by_rank) {
+    rank_sort_kernel<<<(unsigned)((n + kRankBodies - 1) / kRankBodies), kRankWarps * kWarp, 0, s>>>(
+        b.k1, m, x, y, z, n, b.sys_of, b.ss, b.k0, b.v0, b.spos);
+    return;
   }
-}
-
-int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n, int bits,
-                        int32_t *hist, int *err, cudaStream_t s, const int32_t *key_counts,
-                        int64_t n_key_values) {
-  return sort_passes<uint32_t>(k0, v0, k1, v1, n, nullptr, bits, hist, err, false, s, key_counts,
-                               n_key_values);
-}
-
-// The key sort orders all bodies of a batch by key; a stable sort by system
-// then restores the systems' ranges with each range in key order (LSD order:
-// the system is the most significant part of the (system, key) pair).
-void launch_sort_by_system(int64_t n, Buffers &b, cudaStream_t s) {
-  if (b.nsys < 2) return;
-  int bits = 1;
-  while ((1 << bits) < b.nsys) ++bits;
-  uint64_t *ck0 = reinterpret_cast<uint64_t *>(b.cn_quad);       // scratch until the upward pass
-  uint64_t *ck1 = reinterpret_cast<uint64_t *>(b.cn_quad) + b.cap;
-  int32_t *cv0 = b.cn_parent;                                    // scratch until the records
-  int32_t *cv1 = b.bn_flag;                                      // scratch until the marks
-  const int grid = grid_for(n, 256, 148 * 16);
-  sys_keys_kernel<<<grid, 256, 0, s>>>(b.v0, b.sys_of, n, ck0, cv0);
-  radix_sort_pairs(ck0, cv0, ck1, cv1, n, nullptr, bits, b.hist, &b.sc->err, s);
-  regather_kernel<<<grid, 256, 0, s>>>(b.k0, b.v0, cv0, n, b.k1, b.v1);
-  cudaMemcpyAsync(b.k0, b.k1, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
-  cudaMemcpyAsync(b.v0, b.v1, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
-}
-
-void launch_gather(const double *m, const double *x, const double *y, const double *z, int64_t n,
-                   Buffers &b, cudaStream_t s) {
-  gather_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(m, x, y, z, b.v0, n, b.spos);
+  const int passes = plan.kpass + plan.spass;
+  const SortScratch c = sort_scratch(n, passes, b.hist);
+  const bool odd = passes & 1;
+  uint64_t *ki = odd ? b.k1 : b.k0, *ko = odd ? b.k0 : b.k1;
+  int32_t *vi = odd ? b.v1 : b.v0, *vo = odd ? b.v0 : b.v1;
+  for (int p = 0; p < passes; ++p) {
+    // the key's digits, then the system's: every system's bodies end up
+    // together, each range in key order (LSD order)
+    if (p < plan.kpass)
+      one_pass<uint64_t, false>(c, p, n, 8 * p, nullptr, ki, vi, ko, vo, &b.sc->err, s);
+    else
+      one_pass<uint64_t, true>(c, p, n, 8 * (p - plan.kpass), b.sys_of, ki, vi, ko, vo, &b.sc->err, s);
+    uint64_t *tk = ki; ki = ko; ko = tk;
+    int32_t *tv = vi; vi = vo; vo = tv;
+  }
+  gather_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(
+      reinterpret_cast<const double4 *>(b.cn_oct), b.v0, n, b.spos);
 }
 
 }  // namespace bh

@@ -1,0 +1,112 @@
+"""The build's size-dependent paths: keys, permutation, octree records and
+moments against the oracle's Morton tree on both sides of every switch (sort by
+counting / radix passes, one or four binary nodes a thread, staged / per-level
+upward pass), at the edges of their tiles, and with shapes that stress them
+(equal keys, one long chain of nested nodes, shallow trees, odd pass counts)."""
+import numpy as np
+import pytest
+
+from conftest import xyz
+from refcompact import compact_from_reference
+
+pytestmark = pytest.mark.gpu
+
+
+def _cloud(n, seed=0):
+    rng = np.random.default_rng(seed)
+    return rng.uniform(0.5, 1.5, n) / n, rng.normal(size=(n, 3))
+
+
+def _check(oracle_mod, m, q, depth=21, order=4):
+    from hierarquicos_b200.system import BHSystem
+
+    s = BHSystem()
+    s.build(m, *xyz(q), order=order, depth=depth)
+    s.sync()
+    keys, perm = s.keys()
+    ref = oracle_mod.MortonTree(m, *xyz(q), L=depth, ssa=1.2, use_quadrupole=True, fma_mode=1)
+    rkeys, rperm = ref.sorted()
+    assert np.array_equal(keys, rkeys) and np.array_equal(perm, rperm)
+    nodes = s.nodes()
+    _, meta, children, nch = compact_from_reference(ref.nodes())
+    assert np.array_equal(nodes["meta"], meta)
+    used = np.arange(8)[None, :] < nch[:, None]
+    assert np.array_equal(np.where(used, nodes["child"], 0), children)
+    return s, nodes, perm
+
+
+def _moments(m, q, nodes, perm):
+    """Masses, centres and quadrupoles summed over each node's bodies (relative
+    to the sum of the terms' absolute values: n u of rounding on either side)."""
+    ms, qs = m[perm], q[perm]
+    for j in range(len(nodes["meta"])):
+        f, c = nodes["meta"][j][:2]
+        w, r = ms[f:f + c], qs[f:f + c]
+        tol = 4 * (c + 64) * 2.0 ** -53
+        assert abs(nodes["com"][j][3] - w.sum()) <= tol * w.sum()
+        com = (w[:, None] * r).sum(0) / w.sum()
+        assert (np.abs(nodes["com"][j][:3] - com) <= tol * np.abs(w[:, None] * r).sum(0) / w.sum() + 1e-300).all()
+        d = r - com
+        ref = np.array([(w * d[:, a] * d[:, b]).sum() for a, b in ((0, 0), (1, 1), (2, 2), (0, 1), (0, 2), (1, 2))])
+        size = w.sum() * (np.abs(r - com).max() + np.abs(com).max() * 2.0 ** -20) ** 2
+        assert (np.abs(nodes["quad"][j] - ref) <= 1e-9 * size).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 63, 64, 65, 255, 256, 257, 1023, 1025, 2049, 4097])
+def test_small_builds(oracle_mod, n):
+    m, q = _cloud(n, n)
+    if n < 2:
+        from hierarquicos_b200.system import BHSystem
+
+        f = BHSystem().forces(m, *xyz(q)).cpu().numpy()
+        assert (f == 0.0).all()
+        return
+    s, nodes, perm = _check(oracle_mod, m, q)
+    _moments(m, q, nodes, perm)
+    s.close()
+
+
+@pytest.mark.parametrize("n", [16733, 16734, 32769, 65536, 65537, 262144, 262145])
+def test_switches(oracle_mod, n):
+    s, _, _ = _check(oracle_mod, *_cloud(n, 1))
+    s.close()
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 5, 8, 16])
+@pytest.mark.parametrize("n", [3000, 20000])
+def test_depths(oracle_mod, n, depth):
+    """Odd and even numbers of radix passes, and buckets of equal keys."""
+    s, _, _ = _check(oracle_mod, *_cloud(n, 2), depth=depth)
+    s.close()
+
+
+def test_nested_chain(oracle_mod):
+    """Bodies that halve their distance to a corner: every level holds a node
+    that spans almost all bodies (the longest lists of the staged pass)."""
+    rng = np.random.default_rng(4)
+    n = 40000
+    q = rng.uniform(0.5, 1.0, size=(n, 3)) * 2.0 ** -rng.integers(0, 20, size=(n, 1))
+    q = np.concatenate([q, q[:300]])  # and some exact duplicates
+    m = np.full(len(q), 1.0 / len(q))
+    s, nodes, perm = _check(oracle_mod, m, q)
+    s.close()
+
+
+@pytest.mark.parametrize("order", [1, 4, 8])
+def test_batch_equals_lone_systems(order):
+    """Both sorts of a batch, with systems of one body and sizes off every tile:
+    each system's keys and moments are its own build's, bit for bit."""
+    from hierarquicos_b200.system import BHSystem, offsets_of
+
+    for sizes in ([1, 2, 300, 1, 4097, 65], [1, 30000, 257, 2, 25000, 700], [37] * 300 + [22000]):
+        m, q = _cloud(sum(sizes), 9)
+        off = offsets_of(sizes)
+        b = BHSystem()
+        f = b.forces_batch(m, *xyz(q), off, order=order, theta=0.6, eps=0.01).cpu().numpy()
+        lone = BHSystem()
+        for s in range(len(sizes)) if len(sizes) < 10 else [0, 150, 300]:
+            a, e = int(off[s]), int(off[s + 1])
+            g = lone.forces(m[a:e], *xyz(q[a:e]), order=order, theta=0.6, eps=0.01).cpu().numpy()
+            assert np.array_equal(f[3 * a:3 * e], g), (sizes[s], s)
+        b.close()
+        lone.close()
