@@ -150,6 +150,7 @@ finalize_kernel(const double *__restrict__ partials, const RedItem *__restrict__
                 int n_items, double amp, int L, SysScalars *__restrict__ sys, Scalars *sc) {
   __shared__ double red[10];
   __shared__ int range[2];
+  pdl_enter();
   const int s = blockIdx.x;
   if (threadIdx.x == 0) {
     int a = 0, b = n_items;
@@ -229,6 +230,7 @@ keys_kernel(const double *__restrict__ m, const double *__restrict__ x,
             uint64_t *__restrict__ keys, int32_t *__restrict__ vals, double4 *__restrict__ packed,
             int kpass, int spass, uint32_t *__restrict__ counts) {
   __shared__ uint32_t h[RADIX ? kMaxSortPasses : 1][256];
+  pdl_enter();
   if (RADIX) {
     for (int i = threadIdx.x; i < (kpass + spass) * 256; i += 256) (&h[0][0])[i] = 0;
     __syncthreads();
@@ -438,14 +440,14 @@ static void run_keys(const double *m, const double *x, const double *y, const do
   const SortPlan plan = sort_plan(n, L, b);
   const int depth = L == 0 ? kMaxDepth : L;
   if (plan.by_rank) {
-    keys_kernel<CHECK, false><<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(
-        m, x, y, z, n, depth, b.sys_of, b.ss, b.sc, b.k1, nullptr, nullptr, 0, 0, nullptr);
+    launch_pdl(keys_kernel<CHECK, false>, grid_for(n, 256, 148 * 16), 256, 0, s, m, x, y, z, n, depth,
+               b.sys_of, b.ss, b.sc, b.k1, nullptr, nullptr, 0, 0, nullptr);
     return;
   }
   const bool odd = (plan.kpass + plan.spass) & 1;  // the passes end in k0, v0
   cudaMemsetAsync(b.hist, 0, plan.scratch * sizeof(int32_t), s);
-  keys_kernel<CHECK, true><<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(
-      m, x, y, z, n, depth, b.sys_of, b.ss, b.sc, odd ? b.k1 : b.k0, odd ? b.v1 : b.v0,
+  launch_pdl(
+      keys_kernel<CHECK, true>, grid_for(n, 256, 148 * 8), 256, 0, s, m, x, y, z, n, depth, b.sys_of, b.ss, b.sc, odd ? b.k1 : b.k0, odd ? b.v1 : b.v0,
       reinterpret_cast<double4 *>(b.cn_oct), plan.kpass, plan.spass,
       reinterpret_cast<uint32_t *>(b.hist));
 }
@@ -454,8 +456,8 @@ void launch_keys(const double *m, const double *x, const double *y, const double
                  int L, double amp, int com_mode, Buffers &b, cudaStream_t s) {
   cudaMemsetAsync(b.sc, 0, sizeof(Scalars), s);  // batch-wide flags start clear
   reduce_partials<<<b.n_items, kRedThreads, 0, s>>>(m, x, y, z, b.items, com_mode, b.partials);
-  finalize_kernel<<<b.nsys, 320, 0, s>>>(b.partials, b.items, b.n_items, amp,
-                                         L == 0 ? kMaxDepth : L, b.ss, b.sc);
+  launch_pdl(finalize_kernel, b.nsys, 320, 0, s, b.partials, b.items, b.n_items, amp,
+             L == 0 ? kMaxDepth : L, b.ss, b.sc);
   run_keys<true>(m, x, y, z, n, L, b, s);
 }
 

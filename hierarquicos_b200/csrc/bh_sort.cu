@@ -34,10 +34,10 @@ constexpr int kRadix = 256;
 
 // Sum over the systems of n_s^2 up to which a batch is sorted by counting; above
 // it the comparisons cost more than the radix passes.  Whole builds, us, counting
-// / radix: one system of 1,024 bodies 80 / 125, 8,192 109 / 156, 16,384 156 / 161,
-// 20,000 213 / 164; batches (whose radix sort has passes over the system too) of
-// 1.4e8 218 / 298, 6.7e8 352 / 322, 1.5e9 535 / 338.
-constexpr double kRankPairsOne = 2.8e8, kRankPairsBatch = 4e8;
+// / radix: one system of 1,024 bodies 69 / 101, 8,192 110 / 127, 12,000 128 / 131,
+// 16,384 202 / 138; batches (whose radix sort has passes over the system too) of
+// 1.4e8 in 48 systems 159 / 233, in 16 systems 179 / 167, 6.7e8 293 / 269.
+constexpr double kRankPairsOne = 1.44e8, kRankPairsBatch = 2.5e8;
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
@@ -132,8 +132,9 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
   constexpr int kItems = ITEMS;
   constexpr int kTile = ITEMS * kSortThreads;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-  if (threadIdx.x == 0) S.tile = atomicAdd(tile_ctr, 1);
   for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) (&S.wh[0][0])[i] = 0;
+  pdl_enter();
+  if (threadIdx.x == 0) S.tile = atomicAdd(tile_ctr, 1);
   __syncthreads();
   const int t = S.tile;
   const int64_t tile_base = (int64_t)t * kTile;
@@ -256,6 +257,7 @@ scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, i
 __global__ void __launch_bounds__(256)
 gather_kernel(const double4 *__restrict__ packed, const int32_t *__restrict__ perm, int64_t n,
               double4 *__restrict__ spos) {
+  pdl_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     spos[i] = packed[perm[i]];
@@ -291,6 +293,7 @@ rank_sort_kernel(const uint64_t *__restrict__ keys, const double *__restrict__ m
   __shared__ unsigned part[kRankWarps][kRankBodies];
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   const int64_t base = (int64_t)blockIdx.x * kRankBodies;
+  pdl_enter();
   int64_t t[2];
   uint64_t key[2];
   int mine[2];
@@ -363,8 +366,8 @@ void launch_pass(int64_t ntiles, const K *ki, const int32_t *vi, K *ko, int32_t 
                          smem);
     done[dev] = true;
   }
-  onesweep_kernel<K, ITEMS, SYS><<<(unsigned)ntiles, kSortThreads, smem, s>>>(
-      ki, vi, ko, vo, n, shift, sys_of, counts, tiles, ctr, err);
+  launch_pdl(
+      onesweep_kernel<K, ITEMS, SYS>, ntiles, kSortThreads, smem, s, ki, vi, ko, vo, n, shift, sys_of, counts, tiles, ctr, err);
 }
 
 // scratch layout (int32 entries): digit counts [passes][256], tile counters
@@ -446,8 +449,8 @@ void launch_sort(const double *m, const double *x, const double *y, const double
                  int L, Buffers &b, cudaStream_t s) {
   const SortPlan plan = sort_plan(n, L, b);
   if (plan.by_rank) {
-    rank_sort_kernel<<<(unsigned)((n + kRankBodies - 1) / kRankBodies), kRankWarps * kWarp, 0, s>>>(
-        b.k1, m, x, y, z, n, b.sys_of, b.ss, b.k0, b.v0, b.spos);
+    launch_pdl(
+        rank_sort_kernel, (n + kRankBodies - 1) / kRankBodies, kRankWarps * kWarp, 0, s, b.k1, m, x, y, z, n, b.sys_of, b.ss, b.k0, b.v0, b.spos);
     return;
   }
   const int passes = plan.kpass + plan.spass;
@@ -465,8 +468,8 @@ void launch_sort(const double *m, const double *x, const double *y, const double
     uint64_t *tk = ki; ki = ko; ko = tk;
     int32_t *tv = vi; vi = vo; vo = tv;
   }
-  gather_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(
-      reinterpret_cast<const double4 *>(b.cn_oct), b.v0, n, b.spos);
+  launch_pdl(
+      gather_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, reinterpret_cast<const double4 *>(b.cn_oct), b.v0, n, b.spos);
 }
 
 }  // namespace bh

@@ -73,6 +73,7 @@ karras_kernel(const uint64_t *__restrict__ k, int64_t n, const int32_t *__restri
   __shared__ int cnt[kRankRows][kWarp];
   __shared__ int before[kWarp];
   __shared__ int s_tile;
+  pdl_enter();
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
   for (int i = threadIdx.x; i < kRankRows * kWarp; i += kRankThreads) (&cnt[0][0])[i] = 0;
   __syncthreads();
@@ -161,6 +162,7 @@ records_kernel(int64_t n, const int32_t *__restrict__ sys_of, SysScalars *__rest
                int32_t *__restrict__ cparent, int32_t *__restrict__ level_begin,
                int32_t *__restrict__ gflag) {
   __shared__ int begin[kWarp];
+  pdl_enter();
   if (threadIdx.x < kWarp) {
     const int l = threadIdx.x;
     const int c = l <= kMaxDepth ? level_count[l] : 0;
@@ -244,6 +246,7 @@ group_flags_kernel(const int4 *__restrict__ meta, const int32_t *__restrict__ ch
                    const int32_t *__restrict__ cparent, const Scalars *__restrict__ sc, int G,
                    int U, const SysScalars *__restrict__ sys, int nsys,
                    int32_t *__restrict__ gflag) {
+  pdl_enter();
   // every system starts a group (this also covers lone bodies, which have no node)
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nsys; q += gridDim.x * blockDim.x)
     if (sys[q].n > 0) gflag[sys[q].off] = 1;
@@ -289,6 +292,7 @@ group_first_kernel(int64_t n, const int32_t *__restrict__ gflag, Scalars *__rest
                    int32_t *ticket, uint64_t *words, int32_t *__restrict__ g_first) {
   __shared__ int ws[kGroupThreads / kWarp];
   __shared__ int s_tile, s_before;
+  pdl_enter();
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
   __syncthreads();
   const int tile = s_tile;
@@ -363,24 +367,23 @@ void launch_build_tree(int64_t n, int L, Buffers &b, cudaStream_t s) {
   // against 9 us)
   auto run = [&](auto kernel, int items) {
     const int64_t tile = (int64_t)kRankThreads * items;
-    kernel<<<(unsigned)((n + tile - 1) / tile), kRankThreads, 0, s>>>(
-        b.k0, n, b.sys_of, b.ss, b.sc, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
+    launch_pdl(
+        kernel, (n + tile - 1) / tile, kRankThreads, 0, s, b.k0, n, b.sys_of, b.ss, b.sc, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
         b.bn_rank, t.tickets, t.tree_words, t.level_count);
   };
   if (n <= (1 << 18)) run(karras_kernel<1>, 1);
   else run(karras_kernel<4>, 4);
-  records_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(
-      n, b.sys_of, b.ss, b.sc, t.level_count, b.bn_left, b.bn_right, b.bn_first, b.bn_last,
+  launch_pdl(
+      records_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, n, b.sys_of, b.ss, b.sc, t.level_count, b.bn_left, b.bn_right, b.bn_first, b.bn_last,
       b.bn_level, b.bn_rank, b.cn_bin, b.cn_meta, b.cn_child, b.cn_parent, b.level_begin, b.gflag);
 }
 
 void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaStream_t s) {
   const BuildTmp t = build_tmp(n, b);
-  group_flags_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(b.cn_meta, b.cn_child, b.cn_parent,
-                                                                b.sc, group_size, group_span, b.ss,
-                                                                b.nsys, b.gflag);
-  group_first_kernel<<<(unsigned)((n + kGroupTile - 1) / kGroupTile), kGroupThreads, 0, s>>>(
-      n, b.gflag, b.sc, t.tickets + 1, t.group_words, b.g_first);
+  launch_pdl(group_flags_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, b.cn_meta, b.cn_child,
+             b.cn_parent, b.sc, group_size, group_span, b.ss, b.nsys, b.gflag);
+  launch_pdl(
+      group_first_kernel, (n + kGroupTile - 1) / kGroupTile, kGroupThreads, 0, s, n, b.gflag, b.sc, t.tickets + 1, t.group_words, b.g_first);
 }
 
 }  // namespace bh

@@ -102,9 +102,11 @@ __device__ __forceinline__ void add_child(double pm, double px, double py, doubl
 
 // Mass, centre of mass and moments of node j from its children.  For a node
 // with child entries, all child records are loaded before any is used, so the
-// loads overlap; the sums run in child order either way.
-template <int ORDER>
-__device__ void compute_node(int j, const int4 *__restrict__ meta, const int32_t *__restrict__ child,
+// loads overlap; the sums run in child order either way.  WAIT: the previous
+// level's launch may still be running; what it does not write (the records and
+// the lone bodies) is loaded before waiting for it.
+template <int ORDER, bool WAIT>
+__device__ __forceinline__ void compute_node(int j, const int4 *__restrict__ meta, const int32_t *__restrict__ child,
                              const double4 *__restrict__ spos, const int32_t *__restrict__ sys_of,
                              const SysScalars *__restrict__ sys, double4 *com, double *quad,
                              double *oct, float4 *__restrict__ fq, float4 *__restrict__ fo) {
@@ -117,6 +119,7 @@ __device__ void compute_node(int j, const int4 *__restrict__ meta, const int32_t
   double Q[6] = {0, 0, 0, 0, 0, 0};
   double O[14] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (mt.w == 0) {  // bucket of identical keys: its bodies are the children
+    if (WAIT) cudaGridDependencySynchronize();
     for (int c = 0; c < mt.y; ++c) {
       const double4 p = spos[mt.x + c];
       M = M + p.w;
@@ -147,8 +150,12 @@ __device__ void compute_node(int j, const int4 *__restrict__ meta, const int32_t
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       cd[c] = make_double4(0.0, 0.0, 0.0, 0.0);
-      if (c < mt.w) cd[c] = ch[c] < 0 ? spos[~ch[c]] : ld_com(com + ch[c]);
+      if (c < mt.w && ch[c] < 0) cd[c] = spos[~ch[c]];
     }
+    if (WAIT) cudaGridDependencySynchronize();
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c < mt.w && ch[c] >= 0) cd[c] = ld_com(com + ch[c]);
     double Qd[ORDER >= 4 ? 8 : 1][6];
     if (ORDER >= 4) {
 #pragma unroll
@@ -226,9 +233,20 @@ upward_level_kernel(int level, const int32_t *__restrict__ level_begin,
                     const double4 *__restrict__ spos, const int32_t *__restrict__ sys_of,
                     const SysScalars *__restrict__ sys, double4 *com, double *quad, double *oct,
                     float4 *__restrict__ fq, float4 *__restrict__ fo) {
+  // The next level's launch may start now.  The records were complete before
+  // the deepest level's (ordinary) launch began; every thread waits for the level
+  // before this one, which waited for its own predecessor, so the levels complete
+  // in order.
+  cudaTriggerProgrammaticLaunchCompletion();
   const int lb = level_begin[level], le = level_begin[level + 1];
-  for (int j = lb + blockIdx.x * blockDim.x + threadIdx.x; j < le; j += gridDim.x * blockDim.x)
-    compute_node<ORDER>(j, meta, child, spos, sys_of, sys, com, quad, oct, fq, fo);
+  int j = lb + blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= le) {
+    cudaGridDependencySynchronize();
+    return;
+  }
+  compute_node<ORDER, true>(j, meta, child, spos, sys_of, sys, com, quad, oct, fq, fo);
+  for (j += gridDim.x * blockDim.x; j < le; j += gridDim.x * blockDim.x)
+    compute_node<ORDER, false>(j, meta, child, spos, sys_of, sys, com, quad, oct, fq, fo);
 }
 
 // ---- by chunks of bodies ----
@@ -364,6 +382,7 @@ upward_chunk_kernel(UpArgs a) {
   __shared__ unsigned levels;
   const int64_t base = (int64_t)blockIdx.x * kChunk;
   const int64_t i = base + threadIdx.x;
+  pdl_enter();
   if (threadIdx.x == 0) levels = 0;
   int64_t j = -1;
   int lev = -1, nch = 0, bucket = 0;
@@ -449,6 +468,7 @@ upward_list_kernel(UpArgs a, int stage) {
   extern __shared__ __align__(16) unsigned char up_smem[];
   ListEntry *entry = reinterpret_cast<ListEntry *>(up_smem);  // by level
   __shared__ int begin[kWarp + 1], fill[kWarp];
+  pdl_enter();
   int32_t *cnt;
   const int32_t *list = up_list(a, stage, blockIdx.x, cnt);
   const int n = min(*cnt, kListCap);
@@ -560,21 +580,26 @@ void launch_upward_t(const UpArgs &a, cudaStream_t s) {
                          kListCap * (int)sizeof(ListEntry));
     done[dev] = true;
   }
-  upward_chunk_kernel<ORDER><<<(unsigned)((a.n + kChunk - 1) / kChunk), kUpThreads, chunk_smem, s>>>(a);
+  launch_pdl(upward_chunk_kernel<ORDER>, (a.n + kChunk - 1) / kChunk, kUpThreads, chunk_smem, s, a);
   for (int stage = 2; a.n > ((int64_t)1 << (kChunkBits + kStageBits * (stage - 2))); ++stage) {
     const int bits = kChunkBits + kStageBits * (stage - 1);
-    upward_list_kernel<ORDER><<<(unsigned)((a.n + ((int64_t)1 << bits) - 1) >> bits), kUpThreads,
-                                (size_t)bh_min64(kListCap, a.n) * sizeof(ListEntry), s>>>(a, stage);
+    launch_pdl(upward_list_kernel<ORDER>, (a.n + ((int64_t)1 << bits) - 1) >> bits, kUpThreads,
+               (size_t)bh_min64(kListCap, a.n) * sizeof(ListEntry), s, a, stage);
   }
 }
 
 template <int ORDER>
 void launch_levels(int64_t n, Buffers &b, cudaStream_t s) {
   const int grid = grid_for(n / 2 + 1, 128, 148 * 8);
-  for (int level = kMaxDepth; level >= 0; --level)
-    upward_level_kernel<ORDER><<<grid, 128, 0, s>>>(level, b.level_begin, b.cn_meta, b.cn_child,
-                                                    b.spos, b.sys_of, b.ss, b.cn_com, b.cn_quad,
-                                                    b.cn_oct, b.cn_fq, b.cn_fo);
+  for (int level = kMaxDepth; level >= 0; --level) {
+    if (level == kMaxDepth)
+      upward_level_kernel<ORDER><<<grid, 128, 0, s>>>(level, b.level_begin, b.cn_meta, b.cn_child,
+                                                      b.spos, b.sys_of, b.ss, b.cn_com, b.cn_quad,
+                                                      b.cn_oct, b.cn_fq, b.cn_fo);
+    else
+      launch_pdl(upward_level_kernel<ORDER>, grid, 128, 0, s, level, b.level_begin, b.cn_meta,
+                 b.cn_child, b.spos, b.sys_of, b.ss, b.cn_com, b.cn_quad, b.cn_oct, b.cn_fq, b.cn_fo);
+  }
 }
 
 }  // namespace

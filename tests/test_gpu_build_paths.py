@@ -66,7 +66,7 @@ def test_small_builds(oracle_mod, n):
     s.close()
 
 
-@pytest.mark.parametrize("n", [16733, 16734, 32769, 65536, 65537, 262144, 262145])
+@pytest.mark.parametrize("n", [12000, 12001, 32769, 65536, 65537, 262144, 262145])
 def test_switches(oracle_mod, n):
     s, _, _ = _check(oracle_mod, *_cloud(n, 1))
     s.close()
