@@ -30,16 +30,28 @@ namespace bh {
 namespace {
 
 constexpr int64_t kChunk = 512 * 1024;  // bytes per slot
-constexpr int kMaxWorkers = 8;
+// Threads of a transfer: few up to kFewBytes, many above.  Waking threads and
+// their CUDA calls, which take one lock, cost more than a small copy gains.
+// Drop-in calls with pageable arrays (monopole, theta 0.9), us, 3 / 8 threads:
+// 65,536 bodies 575 / 700, 262,147 1340 / 1900, 2^20 4200 / 4740; 4,000,000 20570 /
+// 16700 (2 threads are as good as 3 up to 2^20, 4 vary between 550 and 740 at
+// 65,536; 12 and 16 are slower than 8).  On the 16 cores of one host.
+constexpr int kFewWorkers = 3, kMaxWorkers = 8;
+constexpr int64_t kFewBytes = 48ll << 20;
+constexpr int64_t kMinChunk = 64 * 1024;
 
-// Runs one job at a time on T threads (worker 0 is the calling thread).  The
+// Runs one job at a time on T threads (worker 0 is the calling thread).  A
 // pool lives until the process exits; its threads wait on a condition
 // variable between jobs.
 class WorkerPool {
  public:
-  static WorkerPool &get() {
-    static WorkerPool *pool = new WorkerPool();  // never destroyed: threads outlive static teardown
-    return *pool;
+  static WorkerPool &get(int64_t bytes) {  // never destroyed: threads outlive static teardown
+    if (bytes <= kFewBytes) {
+      static WorkerPool *few = new WorkerPool(kFewWorkers);
+      return *few;
+    }
+    static WorkerPool *many = new WorkerPool(kMaxWorkers);
+    return *many;
   }
   int size() const { return n_; }
   void run(const std::function<void(int)> &fn) {
@@ -58,9 +70,9 @@ class WorkerPool {
   }
 
  private:
-  WorkerPool() {
+  explicit WorkerPool(int most) {
     const unsigned hw = std::thread::hardware_concurrency();
-    n_ = (int)(hw == 0 ? 1 : (hw < (unsigned)kMaxWorkers ? hw : (unsigned)kMaxWorkers));
+    n_ = (int)(hw == 0 ? 1 : (hw < (unsigned)most ? hw : (unsigned)most));
     for (int w = 1; w < n_; ++w) std::thread([this, w] { loop(w); }).detach();
   }
   void loop(int w) {
@@ -96,12 +108,17 @@ struct Piece {
   int64_t bytes;
 };
 
-std::vector<Piece> cut(const double *const *host, double *const *dev, int count, int64_t n) {
+// Pieces of about a worker's share, at most a slot, so that a small transfer
+// still occupies every worker.
+std::vector<Piece> cut(const double *const *host, double *const *dev, int count, int64_t n,
+                       int workers) {
   std::vector<Piece> v;
   const int64_t total = n * (int64_t)sizeof(double);
+  const int64_t share = (total * count / workers + 4095) / 4096 * 4096;
+  const int64_t step = share < kMinChunk ? kMinChunk : (share < kChunk ? share : kChunk);
   for (int a = 0; a < count; ++a)
-    for (int64_t o = 0; o < total; o += kChunk)
-      v.push_back(Piece{(char *)host[a] + o, (char *)dev[a] + o, total - o < kChunk ? total - o : kChunk});
+    for (int64_t o = 0; o < total; o += step)
+      v.push_back(Piece{(char *)host[a] + o, (char *)dev[a] + o, total - o < step ? total - o : step});
   return v;
 }
 
@@ -132,7 +149,7 @@ HostKind host_kind(const void *p) {
 HostCopy *hostcopy_create(int device) {
   HostCopy *h = new HostCopy();
   h->device = device;
-  h->workers = WorkerPool::get().size();
+  h->workers = kMaxWorkers;
   const int W = h->workers;
   bool ok = cudaMallocHost((void **)&h->slots, (size_t)(2 * W) * kChunk) == cudaSuccess &&
             cudaEventCreateWithFlags(&h->start, cudaEventDisableTiming) == cudaSuccess;
@@ -169,12 +186,13 @@ void hostcopy_destroy(HostCopy *h) {
 
 cudaError_t hostcopy_upload(HostCopy *h, const double *const *src, double *const *dst, int count,
                             int64_t n, cudaStream_t st) {
-  const std::vector<Piece> pieces = cut(src, dst, count, n);
+  WorkerPool &pool = WorkerPool::get((int64_t)count * n * (int64_t)sizeof(double));
+  const int W = pool.size();
+  const std::vector<Piece> pieces = cut(src, dst, count, n, W);
   cudaError_t e = cudaEventRecord(h->start, st);  // the device arrays may still be read on st
   if (e != cudaSuccess) return e;
   std::atomic<int> first_err{(int)cudaSuccess};
-  const int W = h->workers;
-  WorkerPool::get().run([&](int w) {
+  pool.run([&](int w) {
     cudaError_t r = cudaSetDevice(h->device);
     if (r == cudaSuccess) r = cudaStreamWaitEvent(h->st[w], h->start, 0);
     int it = 0;
@@ -206,12 +224,13 @@ cudaError_t hostcopy_download(HostCopy *h, double *dst, const double *src, int64
   const double *srcs[1] = {src};
   double *dsts[1] = {dst};
   // pieces with host = dst (written) and dev = src (read)
-  const std::vector<Piece> pieces = cut(dsts, const_cast<double *const *>(srcs), 1, n);
+  WorkerPool &pool = WorkerPool::get(n * (int64_t)sizeof(double));
+  const int W = pool.size();
+  const std::vector<Piece> pieces = cut(dsts, const_cast<double *const *>(srcs), 1, n, W);
   cudaError_t e = cudaEventRecord(h->start, st);  // the result is complete after st's work
   if (e != cudaSuccess) return e;
   std::atomic<int> first_err{(int)cudaSuccess};
-  const int W = h->workers;
-  WorkerPool::get().run([&](int w) {
+  pool.run([&](int w) {
     cudaError_t r = cudaSetDevice(h->device);
     if (r == cudaSuccess) r = cudaStreamWaitEvent(h->st[w], h->start, 0);
     std::vector<size_t> mine;
