@@ -7,7 +7,7 @@
 // extent (rmax 0), a node's children are its child nodes and lone bodies, or,
 // for a node of identical keys, its bodies.
 //
-//  1. rmax (evaluate_rmax :1095-1131), from the leaves up in one launch: the
+//  1. rmax (evaluate_rmax :1095-1131), from the leaves up, level by level: the
 //     largest distance from a node's centre of mass to any child's centre of
 //     mass plus that child's rmax (massless children skipped).
 //  2. Dual traversal (mutual_interaction_walk_* :1133-1402) as a sequence of
@@ -51,6 +51,7 @@ namespace bh {
 namespace {
 
 constexpr int kGenerations = 2 * (kMaxDepth + 2) + 4;  // each generation deepens a pair
+constexpr int kFirstGenerations = 32;  // run before the host looks whether pairs are left
 
 struct Ent {
   const int4 *meta;
@@ -79,58 +80,55 @@ __device__ __forceinline__ int64_t node_child(const Ent &e, int64_t j, int4 mt, 
   return e.n + mt.x + k;
 }
 
-// rmax of node j from its children (evaluate_rmax, octree_default.f90:1095-1131);
-// the children's rmax is read through L2 (ld.cg) because another thread of
-// the same launch may have written it.
-__device__ __forceinline__ double node_rmax(const Ent &e, int j) {
-  const int4 mt = e.meta[j];
-  const double4 c = e.com[j];
-  double r = 0.0;
-  const int k = node_nchild(mt);
-  for (int q = 0; q < k; ++q) {
-    const int64_t ch = node_child(e, j, mt, q);
-    const double4 cc = ent_com(e, ch);
-    if (cc.w == 0.0) continue;
-    const double dx = cc.x - c.x, dy = cc.y - c.y, dz = cc.z - c.z;
-    const double v = sqrt(dx * dx + dy * dy + dz * dz) + (ch < e.n ? __ldcg(e.rmax + ch) : 0.0);
-    if (v > r) r = v;
-  }
-  return r;
-}
-
-__device__ __forceinline__ int node_children_count(const Ent &e, int j) {
-  const int4 mt = e.meta[j];
-  if (mt.w == 0) return 0;
-  int k = 0;
-  for (int q = 0; q < mt.w; ++q) k += e.child[8 * (int64_t)j + q] >= 0 ? 1 : 0;
-  return k;
-}
-
-// All of evaluate_rmax in one launch, bottom-up with an arrival counter per
-// node (the scheme of the upward pass): a thread starts at every node without
-// node children, and the last child to arrive at a parent goes on with it.
-// Every node is computed once, after its children, with the same arithmetic
-// as the level-by-level form.  A chain longer than the deepest tree raises
-// kErrIndex instead of looping.
-__global__ void __launch_bounds__(256)
-rmax_fused_kernel(const Scalars *__restrict__ scr, Ent e, const int32_t *__restrict__ parent,
-                  double *rmax, int32_t *arrive, int *err) {
-  const int M = scr->n_compact;
-  for (int j0 = blockIdx.x * blockDim.x + threadIdx.x; j0 < M; j0 += gridDim.x * blockDim.x) {
-    if (node_children_count(e, j0) != 0) continue;
-    int j = j0;
-    for (int step = 0;; ++step) {
-      if (step > kNumLevels + 1) { atomicOr(err, kErrIndex); break; }
-      rmax[j] = node_rmax(e, j);
-      const int p = parent[j];
-      if (p < 0) break;
-      const int need = node_children_count(e, p);
-      __threadfence();
-      if (atomicAdd(&arrive[p], 1) != need - 1) break;
-      __threadfence();
-      j = p;
+// evaluate_rmax (octree_default.f90:1095-1131), one launch per level, deepest
+// first: rmax of a node is the largest distance from its centre of mass to any
+// child's plus that child's rmax (massless children skipped).  The distances do
+// not depend on the level before, so they are computed while it runs; then the
+// thread waits for it (as the upward pass's levels do) and adds the children's
+// rmax, read through L2.  Bound: latency.  200,003 bodies: 105 us in one bottom-up
+// launch with arrival counters, 93 here.
+__global__ void __launch_bounds__(128)
+rmax_level_kernel(int level, const int32_t *__restrict__ level_begin, Ent e, double *rmax) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int lb = level_begin[level], le = level_begin[level + 1];
+  bool waited = false;
+  for (int j = lb + blockIdx.x * blockDim.x + threadIdx.x; j < le; j += gridDim.x * blockDim.x) {
+    const int4 mt = e.meta[j];
+    const double4 c = e.com[j];
+    double r = 0.0;
+    if (mt.w == 0) {  // a bucket: bodies only
+      for (int q = 0; q < mt.y; ++q) {
+        const double4 cc = e.spos[mt.x + q];
+        if (cc.w == 0.0) continue;
+        const double dx = cc.x - c.x, dy = cc.y - c.y, dz = cc.z - c.z;
+        const double v = sqrt(dx * dx + dy * dy + dz * dz);
+        if (v > r) r = v;
+      }
+    } else {
+      double d[8];
+      int32_t ch[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        ch[q] = q < mt.w ? e.child[8 * (int64_t)j + q] : -1;
+        d[q] = -1.0;  // no child, or a massless one
+        if (q < mt.w) {
+          const double4 cc = ch[q] < 0 ? e.spos[~ch[q]] : e.com[ch[q]];
+          const double dx = cc.x - c.x, dy = cc.y - c.y, dz = cc.z - c.z;
+          if (cc.w != 0.0) d[q] = sqrt(dx * dx + dy * dy + dz * dz);
+        }
+      }
+      if (!waited) cudaGridDependencySynchronize();
+      waited = true;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (d[q] < 0.0) continue;
+        const double v = d[q] + (ch[q] >= 0 ? __ldcg(e.rmax + ch[q]) : 0.0);
+        if (v > r) r = v;
+      }
     }
+    rmax[j] = r;
   }
+  if (!waited) cudaGridDependencySynchronize();  // the levels complete in order
 }
 
 // Every node's quadrupole divided by its mass, once, for the terms that use
@@ -257,6 +255,7 @@ dual_gen_kernel(Ent e, const int2 *__restrict__ fin, const unsigned long long *_
   __shared__ int ws[kGenWarps];
   __shared__ int s_tile;
   __shared__ int64_t s_base[2];
+  pdl_enter();
   // After a frontier overflow the count exceeds what was written and the buffer
   // has slots that no pair was written to (any pair whose outputs did not fit):
   // the later generations take nothing from it, and the host repeats the
@@ -649,8 +648,11 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
   e.quad = b.cn_quad; e.oct = b.cn_oct; e.rmax = d.rmax; e.n = n;
   e.squad = p.order >= 4 ? d.squad : nullptr;
   const int lgrid = grid_for(n / 2 + 1, 256, 148 * 8);
-  cudaMemsetAsync(d.cnt, 0, (ne + 1) * sizeof(int32_t), s);  // arrival counters (M < ne)
-  rmax_fused_kernel<<<lgrid, 256, 0, s>>>(b.sc, e, b.cn_parent, d.rmax, d.cnt, &b.sc->err);
+  const int rgrid = grid_for(n / 2 + 1, 128, 148 * 8);
+  for (int level = kMaxDepth; level >= 0; --level) {
+    if (level == kMaxDepth) rmax_level_kernel<<<rgrid, 128, 0, s>>>(level, b.level_begin, e, d.rmax);
+    else launch_pdl(rmax_level_kernel, rgrid, 128, 0, s, level, b.level_begin, e, d.rmax);
+  }
   if (p.order >= 4)
     spec_quad_kernel<<<lgrid, 256, 0, s>>>(b.sc, b.cn_com, b.cn_quad, d.squad);
 
@@ -658,6 +660,7 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
   // alternating between generations; [4] overflow flags
   unsigned long long *cnt = d.counters;
   unsigned long long h[5] = {0, 0, 0, 0, 0};
+  int last = 0;  // generations run
   if (b.nsys > 16 * n) return 4;
   for (int attempt = 0; attempt < 8; ++attempt) {
     if (grow(d.front, d.front_cap, 2 * d.want_front) != cudaSuccess) return 1;
@@ -672,30 +675,43 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
     cudaMemsetAsync(d.gen_status, 0, (size_t)kGenerations * 2 * max_tiles * sizeof(uint64_t), s);
     cudaMemsetAsync(d.gen_tiles, 0, kGenerations * sizeof(int32_t), s);
     roots_frontier_kernel<<<(b.nsys + 127) / 128, 128, 0, s>>>(b.ss, b.nsys, f0, cnt);
-    for (int g = 0; g < kGenerations; ++g) {
+    // the first kFirstGenerations, and the rest only if pairs are left: an empty
+    // generation is a launch of 2.7 us, and 27 of the 50 hold pairs at 200,003
+    // bodies (theta 0.6); the call went from 2.65 to 2.57 ms with the resident grid
+    // and programmatic launches, to 2.49 without the last 18
+    bool done = false;
+    for (int g = 0; g < kGenerations && !done; ++g) {
       int2 *fi = (g & 1) ? f1 : f0, *fo = (g & 1) ? f0 : f1;
       uint64_t *st = d.gen_status + (int64_t)g * 2 * max_tiles;
-      dual_gen_kernel<<<148 * 8, kGenThreads, 0, s>>>(
-          e, fi, cnt + (g & 1), fcap, fo, cnt + ((g + 1) & 1), fcap, d.mut, cnt + 2 + (g & 1),
-          cnt + 2 + ((g + 1) & 1), d.mut_cap, p.theta2, cnt + 4, st, st + max_tiles,
+      // the resident blocks (they claim tiles until none is left); most of the
+      // generations are small or empty, so the launch itself counts
+      launch_pdl(
+          dual_gen_kernel, 148 * kGenBlocksPerSm, kGenThreads, 0, s, e, fi, cnt + (g & 1), fcap, fo,
+          cnt + ((g + 1) & 1), fcap, d.mut, cnt + 2 + (g & 1), cnt + 2 + ((g + 1) & 1), d.mut_cap, p.theta2, cnt + 4, st, st + max_tiles,
           d.gen_tiles + g, &b.sc->err);
+      if (g + 1 != kFirstGenerations && g + 1 != kGenerations) continue;
+      if (cudaMemcpyAsync(h, d.counters, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                          s) != cudaSuccess ||
+          cudaStreamSynchronize(s) != cudaSuccess)
+        return 2;
+      done = h[(g + 1) & 1] == 0 || (h[4] & 5) != 0;
+      last = g + 1;
     }
-    if (cudaMemcpyAsync(h, d.counters, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                        s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-      return 2;
     if (h[4] & 4) return 3;
     const bool more_front = (h[4] & 1) != 0, more_mut = (h[4] & 2) != 0;
     if (!more_front && !more_mut) {
-      if (h[kGenerations & 1] != 0) return 3;  // the traversal did not close
+      if (h[last & 1] != 0) return 3;  // the traversal did not close
       break;
     }
     if (attempt == 7) return 4;
     if (more_front) d.want_front *= 2;
-    if (more_mut) d.want_mut *= 2;
+    if (more_mut) {  // the count went on past the buffer: room for all of it at once
+      d.want_mut *= 2;
+      while (!more_front && d.want_mut < (int64_t)h[2 + (last & 1)]) d.want_mut *= 2;
+    }
     if (d.want_mut > ((int64_t)1 << 30) || d.want_front > ((int64_t)1 << 30)) return 4;
   }
-  const int64_t np = (int64_t)h[2 + (kGenerations & 1)];
+  const int64_t np = (int64_t)h[2 + (last & 1)];
   const int64_t nh = 2 * np;
   if (grow(d.keys, d.keys_cap, 2 * (nh > 0 ? nh : 1)) != cudaSuccess) return 1;
   if (grow(d.vals, d.vals_cap, 2 * (nh > 0 ? nh : 1)) != cudaSuccess) return 1;

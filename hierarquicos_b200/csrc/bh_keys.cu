@@ -100,8 +100,8 @@ reduce_partials(const double *__restrict__ m, const double *__restrict__ x,
     }
 #pragma unroll
     for (int q = 0; q < kRedBatch; ++q) {
-    if (p0 + q * kRedThreads >= it.end) break;
-    const double a = av[q], b = bv[q], c = cv[q], w = wv[q];
+      if (p0 + q * kRedThreads >= it.end) break;
+      const double a = av[q], b = bv[q], c = cv[q], w = wv[q];
     mn[0] = fmin(mn[0], a); mx[0] = fmax(mx[0], a);
     mn[1] = fmin(mn[1], b); mx[1] = fmax(mx[1], b);
     mn[2] = fmin(mn[2], c); mx[2] = fmax(mx[2], c);

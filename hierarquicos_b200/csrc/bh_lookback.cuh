@@ -27,9 +27,8 @@ __device__ __forceinline__ void st_relaxed(uint64_t *p, uint64_t v) {
 
 // One counter per thread: publishes `count` for tile t (its word at
 // words[t * stride]) and returns the sum of the counts of the tiles before it.
-// kLookWindow earlier words are read at once, so a chain of tiles that are all
-// in flight costs a memory latency per window, not per tile.
-constexpr int kLookWindow = 8;
+// (Reading 4 or 8 earlier words at once made no sort faster, and a pass of 18 M
+// terms 180 instead of 171 us.)
 __device__ __forceinline__ int64_t thread_lookback(uint64_t *words, int t, int stride, int64_t count,
                                                    int *err) {
   uint64_t *word = words + (int64_t)t * stride;
@@ -39,32 +38,15 @@ __device__ __forceinline__ int64_t thread_lookback(uint64_t *words, int t, int s
   }
   st_relaxed(word, kTileAggregate | (uint64_t)count);
   int64_t excl = 0, spins = 0;
-  int j = t - 1;
-  bool open = true;
-  while (open) {
-    uint64_t w[kLookWindow];
-#pragma unroll
-    for (int q = 0; q < kLookWindow; ++q)  // before tile 0 the prefix is an inclusive 0
-      w[q] = j - q >= 0 ? ld_relaxed(words + (int64_t)(j - q) * stride) : kTileInclusive;
-    int seen = 0;
-    bool wait = false;
-#pragma unroll
-    for (int q = 0; q < kLookWindow; ++q) {
-      if (open && !wait) {
-        if ((w[q] & ~kTileValue) == 0) {
-          wait = true;
-        } else {
-          excl += (int64_t)(w[q] & kTileValue);
-          ++seen;
-          if ((w[q] & ~kTileValue) == kTileInclusive) open = false;
-        }
-      }
+  for (int j = t - 1; j >= 0;) {
+    const uint64_t w = ld_relaxed(words + (int64_t)j * stride);
+    if ((w & ~kTileValue) == 0) {
+      if (++spins > kLookbackSpins) { atomicOr(err, kErrTimeout); break; }
+      continue;
     }
-    j -= seen;
-    if (wait && ++spins > kLookbackSpins) {
-      atomicOr(err, kErrTimeout);
-      break;
-    }
+    excl += (int64_t)(w & kTileValue);
+    if ((w & ~kTileValue) == kTileInclusive) break;
+    --j;
   }
   st_relaxed(word, kTileInclusive | (uint64_t)(excl + count));
   return excl;

@@ -102,6 +102,15 @@ count_hist_kernel(const int32_t *__restrict__ count, int64_t n_values, int passe
   }
 }
 
+// Exclusive scan of each pass's 256 digit counts, in place, one block per pass
+// (every block of a pass scanning them itself: 512 systems 22.6 instead of 22.5 ms).
+__global__ void __launch_bounds__(kSortThreads) digit_scan_kernel(uint32_t *counts) {
+  __shared__ int ws[kSortWarps];
+  pdl_enter();
+  uint32_t *c = counts + blockIdx.x * kRadix + threadIdx.x;  // kSortThreads == kRadix
+  *c = (uint32_t)block_excl_scan((int)*c, ws, nullptr);
+}
+
 template <typename K, int ITEMS, bool SYS>
 struct PassSmem {
   K sk[ITEMS * kSortThreads];
@@ -118,14 +127,13 @@ struct PassSmem {
 // keys nobody reads).
 // 3 blocks per SM (80 registers, no spills; the compiler's own choice was 128
 // and 2 blocks): the 181 M-term sort of Dehnen's method 1 ms faster.
-// counts: the pass's 256 digit counts, which every block scans itself.  sys_of
-// given: the digit is the system's (of the body that the value names), not the
+// starts: first place of each of the pass's 256 digits.  SYS: the digit is the system's (of the body that the value names), not the
 // key's.
 template <typename K, int ITEMS, bool SYS>
 __global__ void __launch_bounds__(kSortThreads, 3)
 onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
                 K *__restrict__ kout, int32_t *__restrict__ vout, int64_t n, int shift,
-                const int32_t *__restrict__ sys_of, const uint32_t *__restrict__ counts,
+                const int32_t *__restrict__ sys_of, const uint32_t *__restrict__ starts,
                 uint64_t *__restrict__ tiles, int32_t *__restrict__ tile_ctr, int *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PassSmem<K, ITEMS, SYS> &S = *reinterpret_cast<PassSmem<K, ITEMS, SYS> *>(smem_raw);
@@ -177,7 +185,7 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
   }
   // publish, then look back over the earlier tiles for this digit
   const int64_t excl = thread_lookback(tiles + d, t, kRadix, cnt, err);
-  S.gbase[d] = block_excl_scan((int)counts[d], S.ws, nullptr) + (int)excl;
+  S.gbase[d] = (int)(starts[d] + excl);
   int start = block_excl_scan(cnt, S.ws, nullptr);
   S.tile_start[d] = start;
   __syncthreads();
@@ -424,6 +432,7 @@ int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, in
   cudaMemsetAsync(hist, 0, c.entries * sizeof(int32_t), s);
   count_hist_kernel<<<grid_for(n_key_values, kSortThreads, 148 * 8), kSortThreads, 0, s>>>(
       key_counts, n_key_values, passes, c.counts);
+  launch_pdl(digit_scan_kernel, passes, kSortThreads, 0, s, c.counts);
   uint32_t *ki = k0, *ko = k1;
   int32_t *vi = v0, *vo = v1;
   for (int p = 0; p < passes; ++p) {
@@ -456,6 +465,7 @@ void launch_sort(const double *m, const double *x, const double *y, const double
   const int passes = plan.kpass + plan.spass;
   const SortScratch c = sort_scratch(n, passes, b.hist);
   const bool odd = passes & 1;
+  launch_pdl(digit_scan_kernel, passes, kSortThreads, 0, s, c.counts);
   uint64_t *ki = odd ? b.k1 : b.k0, *ko = odd ? b.k0 : b.k1;
   int32_t *vi = odd ? b.v1 : b.v0, *vo = odd ? b.v0 : b.v1;
   for (int p = 0; p < passes; ++p) {
