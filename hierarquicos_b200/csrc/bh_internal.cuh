@@ -116,6 +116,7 @@ struct Buffers {
   int64_t wstack_cap = 0;   // entries per warp slot
   int64_t wstack_slots = 0; // stacks: the walk launches at most this many one-warp blocks
   int32_t *counters = nullptr;   // [0] group cursor
+  bool cursor_clear = false;     // the build just queued leaves it at 0 for one walk
   unsigned long long *stats = nullptr;  // interaction counters
   Scalars *sc = nullptr;
   Scalars *sc_host = nullptr;    // pinned mirror
@@ -255,8 +256,8 @@ void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n
                     int32_t *total, int32_t *tmp, int *err, cudaStream_t s,
                     int32_t *total2 = nullptr);
 
-void launch_build_tree(int64_t n, int L, Buffers &b, cudaStream_t s);
-// the upward pass's list counters (cleared by launch_build_tree)
+void launch_build_tree(int64_t n, Buffers &b, cudaStream_t s);
+// the upward pass's list counters (cleared with the rest of scan_tmp)
 int32_t *upward_counters(int64_t n, Buffers &b);
 void launch_upward(int64_t n, int L, int order, Buffers &b, cudaStream_t s);
 void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaStream_t s);

@@ -84,8 +84,15 @@ __device__ __forceinline__ uint64_t key_of(double x, double y, double z, const d
 __global__ void __launch_bounds__(kRedThreads)
 reduce_partials(const double *__restrict__ m, const double *__restrict__ x,
                 const double *__restrict__ y, const double *__restrict__ z,
-                const RedItem *__restrict__ items, int com_mode, double *__restrict__ partials) {
+                const RedItem *__restrict__ items, int com_mode, double *__restrict__ partials,
+                int32_t *__restrict__ clear, int64_t n_clear, Scalars *sc) {
   __shared__ double s[10][kRedThreads];
+  // the first kernel of a build: clears the tree passes' scratch and the flags
+  for (int64_t i = (int64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n_clear;
+       i += (int64_t)gridDim.x * kRedThreads)
+    clear[i] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(Scalars) / sizeof(int))
+    reinterpret_cast<int *>(sc)[threadIdx.x] = 0;
   const RedItem it = items[blockIdx.x];
   double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
@@ -454,8 +461,8 @@ static void run_keys(const double *m, const double *x, const double *y, const do
 
 void launch_keys(const double *m, const double *x, const double *y, const double *z, int64_t n,
                  int L, double amp, int com_mode, Buffers &b, cudaStream_t s) {
-  cudaMemsetAsync(b.sc, 0, sizeof(Scalars), s);  // batch-wide flags start clear
-  reduce_partials<<<b.n_items, kRedThreads, 0, s>>>(m, x, y, z, b.items, com_mode, b.partials);
+  reduce_partials<<<b.n_items, kRedThreads, 0, s>>>(m, x, y, z, b.items, com_mode, b.partials,
+                                                    b.scan_tmp, build_tmp_entries(n), b.sc);
   launch_pdl(finalize_kernel, b.nsys, 320, 0, s, b.partials, b.items, b.n_items, amp,
              L == 0 ? kMaxDepth : L, b.ss, b.sc);
   run_keys<true>(m, x, y, z, n, L, b, s);
@@ -481,6 +488,7 @@ void launch_adopt_seq_com(Buffers &b, cudaStream_t s) {
 
 void launch_keys_only(const double *m, const double *x, const double *y, const double *z, int64_t n,
                       int L, Buffers &b, cudaStream_t s) {
+  cudaMemsetAsync(b.scan_tmp, 0, build_tmp_entries(n) * sizeof(int32_t), s);
   run_keys<false>(m, x, y, z, n, L, b, s);
 }
 

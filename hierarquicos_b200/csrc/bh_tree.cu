@@ -152,6 +152,8 @@ karras_kernel(const uint64_t *__restrict__ k, int64_t n, const int32_t *__restri
 // Octree records, one thread per binary node: node id = nodes of the shallower
 // levels + rank.  Also clears the group flags, and writes the roots, the level
 // starts and the node count.
+// (Marking the groups' first bodies here as well, from the children's ranges,
+// took it from 167 to 450 us at 5,000,011 bodies, to save a launch of 15.)
 __global__ void __launch_bounds__(256)
 records_kernel(int64_t n, const int32_t *__restrict__ sys_of, SysScalars *__restrict__ sys,
                Scalars *__restrict__ sc, const int32_t *__restrict__ level_count,
@@ -289,11 +291,13 @@ static_assert(kGroupTile == kGroupScanTile, "build_tmp_entries in bh_internal.cu
 // blocks write g_first themselves (instead of a scan array and a pass over it).
 __global__ void __launch_bounds__(kGroupThreads)
 group_first_kernel(int64_t n, const int32_t *__restrict__ gflag, Scalars *__restrict__ sc,
-                   int32_t *ticket, uint64_t *words, int32_t *__restrict__ g_first) {
+                   int32_t *__restrict__ cursor, int32_t *ticket, uint64_t *words,
+                   int32_t *__restrict__ g_first) {
   __shared__ int ws[kGroupThreads / kWarp];
   __shared__ int s_tile, s_before;
   pdl_enter();
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;  // of the first walk
   __syncthreads();
   const int tile = s_tile;
   const int64_t base = (int64_t)tile * kGroupTile;
@@ -338,7 +342,8 @@ group_first_kernel(int64_t n, const int32_t *__restrict__ gflag, Scalars *__rest
 
 // Scratch of the tree and group passes in b.scan_tmp (int32 entries): [0], [1]
 // the two tickets, then the nodes of every level, the words of the two
-// look-backs, and the upward pass's list counters; cleared once per build.
+// look-backs, and the upward pass's list counters; cleared by the build's first
+// kernel.
 struct BuildTmp {
   int32_t *tickets, *level_count;
   uint64_t *tree_words, *group_words;
@@ -358,32 +363,32 @@ int32_t *upward_counters(int64_t n, Buffers &b) {
   return reinterpret_cast<int32_t *>(build_tmp(n, b).group_words + (n + kGroupScanTile - 1) / kGroupScanTile);
 }
 
-void launch_build_tree(int64_t n, int L, Buffers &b, cudaStream_t s) {
-  (void)L;
+void launch_build_tree(int64_t n, Buffers &b, cudaStream_t s) {
   const BuildTmp t = build_tmp(n, b);
-  cudaMemsetAsync(b.scan_tmp, 0, build_tmp_entries(n) * sizeof(int32_t), s);
   // one binary node a thread while the tiles all run at once, four above (fewer
   // tiles to look back over: 2^20 bodies 85 against 107 us; 1,024 bodies 20
-  // against 9 us)
-  auto run = [&](auto kernel, int items) {
-    const int64_t tile = (int64_t)kRankThreads * items;
-    launch_pdl(
-        kernel, (n + tile - 1) / tile, kRankThreads, 0, s, b.k0, n, b.sys_of, b.ss, b.sc, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
+  // against 9 us).  The large one is launched ordinarily: started while the
+  // gather drains, it and the records after it took 65 us longer at 5,000,011.
+  if (n <= (1 << 18))
+    launch_pdl(karras_kernel<1>, (n + kRankThreads - 1) / kRankThreads, kRankThreads, 0, s, b.k0, n,
+               b.sys_of, b.ss, b.sc, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
+               b.bn_rank, t.tickets, t.tree_words, t.level_count);
+  else
+    karras_kernel<4><<<(unsigned)((n + 4 * kRankThreads - 1) / (4 * kRankThreads)), kRankThreads, 0, s>>>(
+        b.k0, n, b.sys_of, b.ss, b.sc, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level,
         b.bn_rank, t.tickets, t.tree_words, t.level_count);
-  };
-  if (n <= (1 << 18)) run(karras_kernel<1>, 1);
-  else run(karras_kernel<4>, 4);
-  launch_pdl(
-      records_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, n, b.sys_of, b.ss, b.sc, t.level_count, b.bn_left, b.bn_right, b.bn_first, b.bn_last,
-      b.bn_level, b.bn_rank, b.cn_bin, b.cn_meta, b.cn_child, b.cn_parent, b.level_begin, b.gflag);
+  launch_pdl(records_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, n, b.sys_of, b.ss, b.sc,
+             t.level_count, b.bn_left, b.bn_right, b.bn_first, b.bn_last, b.bn_level, b.bn_rank,
+             b.cn_bin, b.cn_meta, b.cn_child, b.cn_parent, b.level_begin, b.gflag);
 }
 
 void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaStream_t s) {
   const BuildTmp t = build_tmp(n, b);
   launch_pdl(group_flags_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, b.cn_meta, b.cn_child,
              b.cn_parent, b.sc, group_size, group_span, b.ss, b.nsys, b.gflag);
-  launch_pdl(
-      group_first_kernel, (n + kGroupTile - 1) / kGroupTile, kGroupThreads, 0, s, n, b.gflag, b.sc, t.tickets + 1, t.group_words, b.g_first);
+  launch_pdl(group_first_kernel, (n + kGroupTile - 1) / kGroupTile, kGroupThreads, 0, s, n, b.gflag,
+             b.sc, b.counters, t.tickets + 1, t.group_words, b.g_first);
+  b.cursor_clear = true;
 }
 
 }  // namespace bh

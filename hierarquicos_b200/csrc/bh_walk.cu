@@ -935,6 +935,7 @@ template <typename T, int ORDER, int MAXTPL, bool SOFT>
 __global__ void __launch_bounds__(kWarp, walk_min_blocks<T, ORDER>())
 group_walk_kernel(WalkArgs a) {
   __shared__ WarpSmem<T, ORDER> S;
+  pdl_enter();
   const int lane = threadIdx.x;
   int32_t *stack = a.stack + (int64_t)blockIdx.x * a.stack_cap;
   const int stack_cap = (int)a.stack_cap;
@@ -1147,6 +1148,7 @@ __global__ void __launch_bounds__(wide_threads<CONS>(), wide_blocks<CONS>())
 wide_walk_kernel(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char wide_smem_raw[];
   constexpr unsigned kSlots = WideSmem<T, ORDER, CONS>::kSlots;
+  pdl_enter();
   WideSmem<T, ORDER, CONS> &P = *reinterpret_cast<WideSmem<T, ORDER, CONS> *>(wide_smem_raw);
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x & (kWarp - 1);
   if (threadIdx.x == 0) {
@@ -1756,7 +1758,7 @@ static void launch_wide_walk(const WalkArgs &a, cudaStream_t s) {
   const int per = resident_blocks(per_sm, wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS>,
                                   wide_threads<CONS>(), smem);
   const int64_t blocks = bh_min64(a.slots, (int64_t)sm_count() * per);  // one stack per block
-  wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS><<<(unsigned)blocks, wide_threads<CONS>(), smem, s>>>(a);
+  launch_pdl(wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS>, blocks, wide_threads<CONS>(), smem, s, a);
 }
 
 // Which walk a launch takes (pipeline 1).  Few groups leave most of the chip
@@ -1803,7 +1805,7 @@ static void launch_group_walk(const WalkArgs &a, cudaStream_t s) {
   static int per_sm[64] = {};
   const int per = resident_blocks(per_sm, group_walk_kernel<T, ORDER, MAXTPL, SOFT>, kWarp, 0);
   const int64_t blocks = bh_min64(a.slots, (int64_t)sm_count() * per);  // one stack per block
-  group_walk_kernel<T, ORDER, MAXTPL, SOFT><<<(unsigned)blocks, kWarp, 0, s>>>(a);
+  launch_pdl(group_walk_kernel<T, ORDER, MAXTPL, SOFT>, blocks, kWarp, 0, s, a);
 }
 
 static WalkArgs make_args(int64_t n, const WalkParams &p, Buffers &b, double *out) {
@@ -1835,7 +1837,9 @@ static void launch_walk_t(const WalkArgs &a, bool two, bool soft, cudaStream_t s
 
 void launch_walk(int64_t n, const WalkParams &p, Buffers &b, double *out, cudaStream_t s) {
   WalkArgs a = make_args(n, p, b, out);
-  cudaMemsetAsync(b.counters, 0, sizeof(int32_t), s);
+  // the first walk after a build finds the cursor cleared and follows it directly
+  if (!b.cursor_clear) cudaMemsetAsync(b.counters, 0, sizeof(int32_t), s);
+  b.cursor_clear = false;
   const bool two = p.group_size > 32;
   const bool soft = p.eps2 > 0.0;
   if (p.precision == BH_PREC_FP64) {
