@@ -199,29 +199,22 @@ class ClockSampler:
 
 
 def launches_per_evaluation(n, nsys=1, L=21):
-    """Our kernel launches in one build + walk (the pipeline's launch
-    sequence: 54 for one system of 2^20 bodies)."""
-    scan = 1                                           # one chained-scan launch
-
-    def sort(bits):                                    # digit histograms, their scan, passes
-        return 2 + math.ceil(bits / 8)
-
+    """Our kernel launches in one build + walk of nsys equal systems (the
+    pipeline's launch sequence: 40 for one system of 2^20 bodies)."""
     keys = 3                                           # reduce, finalize, keys
-    particle_sort = sort(3 * L)
-    by_system = 0
-    if nsys >= 2:
-        by_system = 1 + sort(max(1, math.ceil(math.log2(nsys)))) + 1
-    first_bits = 1
-    while (1 << first_bits) <= n:
-        first_bits += 1
-    node_sort = sort(first_bits + 5)
-    # karras, mark, scan (also writes the node count), compact keys, node sort, bin2cn,
-    # records, levels, roots
-    tree = 2 + scan + 1 + node_sort + 1 + 1 + 1 + 1
-    upward = 22                                        # one launch per level
-    groups = 1 + scan + 1                              # flags (and system starts), scan, first
+    if n * n / nsys <= (1.44e8 if nsys == 1 else 2.5e8):
+        sort = 1                                       # places by counting
+    else:                                              # digit scan, passes, gather
+        spass = math.ceil(math.log2(nsys) / 8) if nsys > 1 else 0
+        sort = 1 + math.ceil(3 * L / 8) + spass + 1
+    tree = 2                                           # radix tree with ranks, records
+    if n > 65536:
+        upward = 22                                    # one launch per level
+    else:                                              # chunks, then the lists
+        upward = 1 + (n > 256) + (n > 32768)
+    groups = 2                                         # flags, group starts
     walk = 1
-    return keys + particle_sort + by_system + 1 + tree + upward + groups + walk
+    return keys + sort + tree + upward + groups + walk
 
 
 def dist_max(x, dev, world):
@@ -496,7 +489,7 @@ def run_ours(args):
                 traffic = json.load(fh).get("bytes_per_launch_scaled")
         line["roofline"] = {
             "bound": "fp32",
-            "kernel": "pipe_walk_kernel" if p.pipeline and args.precision == 0 else "group_walk_kernel",
+            "kernel": "team_walk_kernel" if p.pipeline and args.precision == 0 else "group_walk_kernel",
             "achieved": achieved,
             "peak": fp32_peak / 1e3, "unit": "TFLOP/s", "frac": achieved / (fp32_peak / 1e3),
             "traffic": traffic,
