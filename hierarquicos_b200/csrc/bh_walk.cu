@@ -1260,7 +1260,7 @@ wide_walk_kernel(WalkArgs a) {
 // the batches and writes the forces: the batches, order and arithmetic of the
 // one-warp walk, so the same bits.  The consumers (warpgroup 0) take registers
 // over from the producers (warpgroup 1) with setmaxnreg.
-// Bound: the FP32 FMA pipe (64 % busy at 2^20 bodies; the evaluation loop alone
+// Bound: the FP32 FMA pipe (66 % busy at 524,288 bodies; the evaluation loop alone
 // reaches 84 % with 2-5 warps per scheduler, and the producers' instructions
 // take the difference).  2^20 Hernquist bodies 5.20 -> 5.17 ms, 5,000,011 in a
 // uniform sphere 7.00 -> 6.76 ms with the walk's gathered candidates and
