@@ -343,12 +343,15 @@ bh::WalkParams walk_params(const bh_params *p, int order) {
   return w;
 }
 
-// the walk of the whole batch, enqueued without host synchronisation
-int enqueue_walk(bh_system *s, const bh_params *p, double *d_out, cudaStream_t st) {
+// the walk of the whole batch, enqueued without host synchronisation; after_build:
+// the caller has just enqueued the build on st
+int enqueue_walk(bh_system *s, const bh_params *p, double *d_out, cudaStream_t st,
+                 bool after_build = false) {
   ++s->walks_enqueued;
   bh::WalkParams w = walk_params(p, s->order);
   w.g_begin = s->walk_g0;
   w.g_end = s->walk_g1;
+  w.after_build = after_build;
   if (w.count_stats) cudaMemsetAsync(s->b.stats, 0, 4 * sizeof(unsigned long long), st);
   if (p->precision == BH_PREC_DEHNEN) {
     switch (bh::run_dehnen(s->n, w, s->b, s->dehnen, d_out, st)) {
@@ -631,7 +634,7 @@ int bh_system_build_batch(bh_system *s, const double *d_m, const double *d_x,
 // The walk over target groups [g0, g1) (g1 < 0: all), remembered so that a
 // repeated walk (strict-key rebuild, stack growth) covers the same groups.
 static int walk_impl(bh_system *s, const bh_params *p, int g0, int g1, double *d_out,
-                     void *stream) {
+                     void *stream, bool after_build = false) {
   if (!s) return set_err(BH_ERR_INVALID, "sys is NULL");
   if (!s->built) return set_err(BH_ERR_NOT_BUILT, "walk before build");
   int rc = check_params(p, s->n);
@@ -641,7 +644,7 @@ static int walk_impl(bh_system *s, const bh_params *p, int g0, int g1, double *d
   BH_CUDA(cudaSetDevice(s->device));
   s->walk_g0 = g0;
   s->walk_g1 = g1;
-  rc = enqueue_walk(s, p, d_out, (cudaStream_t)stream);
+  rc = enqueue_walk(s, p, d_out, (cudaStream_t)stream, after_build);
   if (rc) return rc;
   BH_CUDA(cudaGetLastError());
   s->walked = 1;
@@ -677,7 +680,7 @@ int bh_system_forces(bh_system *s, const double *d_m, const double *d_x, const d
                      void *stream) {
   int rc = bh_system_build(s, d_m, d_x, d_y, d_z, n, p, stream);
   if (rc) return rc;
-  rc = bh_system_walk(s, p, d_out, stream);
+  rc = walk_impl(s, p, 0, -1, d_out, stream, true);
   if (rc) return rc;
   return finish(s, (cudaStream_t)stream);
 }
@@ -687,7 +690,7 @@ int bh_system_forces_batch(bh_system *s, const double *d_m, const double *d_x,
                            int nsys, const bh_params *p, double *d_out, void *stream) {
   int rc = bh_system_build_batch(s, d_m, d_x, d_y, d_z, offsets, nsys, p, stream);
   if (rc) return rc;
-  rc = bh_system_walk(s, p, d_out, stream);
+  rc = walk_impl(s, p, 0, -1, d_out, stream, true);
   if (rc) return rc;
   return finish(s, (cudaStream_t)stream);
 }
@@ -713,7 +716,7 @@ int bh_system_capture(bh_system *s, const bh_params *p, double *d_out) {
   cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     enqueue_build(s, 0, cap);
-    (void)enqueue_walk(s, p, d_out, cap);
+    (void)enqueue_walk(s, p, d_out, cap, true);
     e = cudaStreamEndCapture(cap, &g);
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&s->graph, g, 0);
@@ -869,7 +872,7 @@ int bh_compute_forces_ex(const double *m, const double *x, const double *y, cons
   Buffers &b = s->b;
   rc = bh_system_build(s, b.hm, b.hx, b.hy, b.hz, n, p, stream);
   if (rc) return rc;
-  rc = bh_system_walk(s, p, b.hout, stream);
+  rc = walk_impl(s, p, 0, -1, b.hout, stream, true);
   if (rc) return rc;
   if (ok != bh::HostKind::kPinned) {
     // pageable result: the status first (it may redo the walk), then the

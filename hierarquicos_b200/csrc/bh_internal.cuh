@@ -116,7 +116,6 @@ struct Buffers {
   int64_t wstack_cap = 0;   // entries per warp slot
   int64_t wstack_slots = 0; // stacks: the walk launches at most this many one-warp blocks
   int32_t *counters = nullptr;   // [0] group cursor
-  bool cursor_clear = false;     // the build just queued leaves it at 0 for one walk
   unsigned long long *stats = nullptr;  // interaction counters
   Scalars *sc = nullptr;
   Scalars *sc_host = nullptr;    // pinned mirror
@@ -277,6 +276,10 @@ struct WalkParams {
   int mac;         // 0 box distance, 1 box distance or every member's own MAC
   int pipeline = 0;  // FP32 walk: 0 one warp per group, 1 producer/consumer warps
   int g_begin = 0, g_end = -1;  // target groups walked: [g_begin, g_end), g_end < 0 = all
+  // The walk directly follows a build in the same stream or graph, which left the
+  // group cursor at 0.  Only a call that queues both may say so: any other walk may
+  // run after one that moved the cursor (a replay, an earlier run of a captured walk).
+  bool after_build = false;
 };
 // Work buffers of Dehnen's dual-tree method (allocated on first use, grown on
 // demand): entity arrays for nodes and bodies (2n entities), the pair

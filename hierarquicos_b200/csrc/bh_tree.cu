@@ -297,7 +297,7 @@ group_first_kernel(int64_t n, const int32_t *__restrict__ gflag, Scalars *__rest
   __shared__ int s_tile, s_before;
   pdl_enter();
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;  // of the first walk
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;  // for a walk queued with the build
   __syncthreads();
   const int tile = s_tile;
   const int64_t base = (int64_t)tile * kGroupTile;
@@ -388,7 +388,6 @@ void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaSt
              b.cn_parent, b.sc, group_size, group_span, b.ss, b.nsys, b.gflag);
   launch_pdl(group_first_kernel, (n + kGroupTile - 1) / kGroupTile, kGroupThreads, 0, s, n, b.gflag,
              b.sc, b.counters, t.tickets + 1, t.group_words, b.g_first);
-  b.cursor_clear = true;
 }
 
 }  // namespace bh

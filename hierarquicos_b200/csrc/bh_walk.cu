@@ -1837,9 +1837,7 @@ static void launch_walk_t(const WalkArgs &a, bool two, bool soft, cudaStream_t s
 
 void launch_walk(int64_t n, const WalkParams &p, Buffers &b, double *out, cudaStream_t s) {
   WalkArgs a = make_args(n, p, b, out);
-  // the first walk after a build finds the cursor cleared and follows it directly
-  if (!b.cursor_clear) cudaMemsetAsync(b.counters, 0, sizeof(int32_t), s);
-  b.cursor_clear = false;
+  if (!p.after_build) cudaMemsetAsync(b.counters, 0, sizeof(int32_t), s);
   const bool two = p.group_size > 32;
   const bool soft = p.eps2 > 0.0;
   if (p.precision == BH_PREC_FP64) {
