@@ -245,8 +245,9 @@ keys_kernel(const double *__restrict__ m, const double *__restrict__ x,
   int bad = 0, amb_any = 0;
   for (int64_t p0 = (int64_t)blockIdx.x * 256; p0 < n; p0 += (int64_t)gridDim.x * 256) {
     const int64_t p = p0 + threadIdx.x;
+    int32_t s = 0;
     if (p < n) {
-      const int32_t s = sys_of[p];
+      s = sys_of[p];
       SysScalars *ss = sys + s;
       const double com[3] = {ss->com[0], ss->com[1], ss->com[2]};
       const double vcen[3] = {ss->vcen[0], ss->vcen[1], ss->vcen[2]};
@@ -260,18 +261,23 @@ keys_kernel(const double *__restrict__ m, const double *__restrict__ x,
         vals[p] = (int32_t)p;
         packed[p] = make_double4(px, py, pz, m[p]);
         for (int q = 0; q < kpass; ++q) atomicAdd(&h[q][(k >> (8 * q)) & 0xff], 1u);
-        if (spass) {  // neighbours share their system: one add per warp
-          const unsigned act = __activemask();
-          int same;
-          __match_all_sync(act, s, &same);
-          if (!same || (threadIdx.x & (kWarp - 1)) == 0)
-            for (int q = 0; q < spass; ++q)
-              atomicAdd(&h[kpass + q][(s >> (8 * q)) & 0xff], same ? (uint32_t)__popc(act) : 1u);
-        }
       }
       if (CHECK && amb && ss->n > 1) {
         ss->key_ambiguous = 1;  // every writer stores the same value
         amb_any = 1;
+      }
+    }
+    if (RADIX && spass) {
+      // Neighbours share their system: one add per warp, by lane 0 for all the
+      // warp's bodies.  The lanes come from the body count, not from which of
+      // them the branches above left together.
+      const unsigned act = __ballot_sync(0xffffffffu, p < n);
+      if (p < n) {
+        int same;
+        __match_all_sync(act, s, &same);
+        if (!same || (threadIdx.x & (kWarp - 1)) == 0)
+          for (int q = 0; q < spass; ++q)
+            atomicAdd(&h[kpass + q][(s >> (8 * q)) & 0xff], same ? (uint32_t)__popc(act) : 1u);
       }
     }
   }

@@ -110,3 +110,40 @@ def test_batch_equals_lone_systems(order):
             assert np.array_equal(f[3 * a:3 * e], g), (sizes[s], s)
         b.close()
         lone.close()
+
+
+@pytest.mark.parametrize("sizes", [[20001, 7, 20000, 1, 33], [1, 2, 3] * 90 + [30001, 31, 17, 45],
+                                   [257, 1, 2000, 63] * 300 + [5, 9001]])
+def test_batch_radix_places(sizes):
+    """Batches above the counting sort's limit, one and two digits of the system:
+    every body has its own place, in its system's range and in that system's key
+    order (a lone build's, by the counting sort where it is small).  Half of the
+    bodies lie on cell edges, so that the lanes of a warp take different ways
+    through the keys kernel before they count their systems."""
+    from hierarquicos_b200.system import BHSystem, offsets_of
+
+    n = sum(sizes)
+    assert sum(k * k for k in sizes) > 5e8
+    rng = np.random.default_rng(6)
+    q = rng.uniform(-1, 1, size=(n, 3))
+    edge = rng.random(n) < 0.5
+    q[edge] = np.round(q[edge] * 32) / 32
+    m = np.full(n, 1.0 / n)
+    off = offsets_of(sizes)
+    b, lone = BHSystem(), BHSystem()
+    b.build_batch(m, *xyz(q), off, strict_keys=0)
+    b.sync()
+    keys, perm = b.keys()
+    assert np.array_equal(np.sort(perm), np.arange(n))
+    system_of = np.repeat(np.arange(len(sizes)), sizes)
+    assert np.array_equal(system_of[perm], system_of)
+    for s in range(0, len(sizes), max(1, len(sizes) // 40)):
+        a, e = int(off[s]), int(off[s + 1])
+        if e - a < 2:
+            continue
+        lone.build(m[a:e], *xyz(q[a:e]), strict_keys=0)
+        lone.sync()
+        k1, p1 = lone.keys()
+        assert np.array_equal(keys[a:e], k1) and np.array_equal(perm[a:e] - a, p1), s
+    b.close()
+    lone.close()
