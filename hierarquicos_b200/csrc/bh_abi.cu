@@ -248,9 +248,17 @@ int set_layout(bh_system *s, const int64_t *off, int nsys, cudaStream_t st) {
   BH_CUDA(cudaMemcpyAsync(b.items, items, (size_t)k * sizeof(bh::RedItem), cudaMemcpyHostToDevice, st));
   b.n_items = k;
   b.nsys = nsys;
-  b.sort_pairs = 0;
+  b.sort_pairs = b.walk_groups[0] = b.walk_groups[1] = 0.0;
+  b.largest = 0;
   for (int q = 0; q < nsys; ++q)
-    b.sort_pairs += (double)(off[q + 1] - off[q]) * (double)(off[q + 1] - off[q]);
+    if (off[q + 1] - off[q] > b.largest) b.largest = off[q + 1] - off[q];
+  for (int q = 0; q < nsys; ++q) {
+    const int64_t k = off[q + 1] - off[q];
+    const double length = sqrt((double)k / (double)b.largest);
+    b.sort_pairs += (double)k * (double)k;
+    b.walk_groups[0] += length * (double)((k + 31) / 32);
+    b.walk_groups[1] += length * (double)((k + 63) / 64);
+  }
   bh::launch_layout(b, st);
   if (items == s->items_pin) {
     if (!s->layout_ev) BH_CUDA(cudaEventCreateWithFlags(&s->layout_ev, cudaEventDisableTiming));

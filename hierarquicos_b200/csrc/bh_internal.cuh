@@ -73,6 +73,8 @@ struct Buffers {
   // batch layout
   int nsys = 0;
   double sort_pairs = 0;           // sum of n_s^2 over the systems
+  int64_t largest = 0;             // bodies of the largest system
+  double walk_groups[2] = {0, 0};  // target groups (32 / 64 bodies) weighed by their walk's length
   SysScalars *ss = nullptr;        // nsys entries
   SysScalars *ss_host = nullptr;   // host mirror
   int32_t *sys_of = nullptr;       // system of each body (same in input and key order)

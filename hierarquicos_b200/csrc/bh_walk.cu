@@ -117,7 +117,9 @@ struct WalkArgs {
   double theta2, G, eps2;
   int out_kind, leaf_cap, count_stats, mac;
   int g_begin, g_end;  // groups walked: [g_begin, g_end), g_end < 0 = all
-  int pipeline;        // FP32: producer/consumer warp teams
+  int pipeline;        // producer / consumer warps
+  int64_t largest;     // choose_walk: bodies of the largest system,
+  double walk_groups;  // and groups weighed by the length of their walks
 };
 
 // a predicated shared-memory store: no branch, whatever the lanes decide
@@ -985,7 +987,7 @@ group_walk_kernel(WalkArgs a) {
 // 7 consumers a block: N = 1,024 81 -> 30 us, 4,096 196 -> 79 us, 16,384 371 ->
 // 157 us against one team (below) per group; the FP64 walk at 65,536 bodies
 // (3 consumers, 4 blocks per SM) 2.37 -> 1.16 ms against one warp per group
-// evaluating its own batches.  launch_group_walk has the sizes where each wins.
+// evaluating its own batches.  choose_walk has the sizes where each wins.
 
 constexpr long long kWaitCycles = 4000000000LL;
 constexpr int kRingStart = 1, kRingCells = 2, kRingBodies = 3, kRingEnd = 4, kRingQuit = 5;
@@ -1761,47 +1763,82 @@ static void launch_wide_walk(const WalkArgs &a, cudaStream_t s) {
   launch_pdl(wide_walk_kernel<T, ORDER, MAXTPL, SOFT, CONS>, blocks, wide_threads<CONS>(), smem, s, a);
 }
 
-// Which walk a launch takes (pipeline 1).  Few groups leave most of the chip
-// idle, so the more warps share a group the better, until the producers fall
-// short; a team's two warps per group fill the chip from about 1,000 groups on.
-// Walk times in us, 7 consumers / 3 consumers / teams (theta 0.5, Plummer):
-//   quadrupole  16,384: 157 / 189 / 371   24,000: 233 / 214 / 420
-//               65,536: 579 / 444 / 516  100,003: 865 / 671 / 549
-//   monopole    16,384: 148 / 159 / 259   65,536: 544 / 350 / 326
-//   octupole    16,384: 235 / 381 / 491   49,152: 682 / 730 / 707
-//               65,536: 925 / 965 / 788
-//   FP64 quad   16,384: 207 / 317 / -     24,000: 301 / 338 / -
-//               32,768: 375 / 374 / -    100,003: 1095 / 1048 / -
-//   FP64 oct    16,384: 398 / 666 / -    100,003: 2257 / 2363 / -
-// (uniform spheres cross at the same sizes within a third).  The octupole, whose
-// batches take longest, never does better with 3 consumers.
-template <typename T, int ORDER> constexpr int64_t seven_max() {
-  return ORDER >= 8 ? INT64_MAX : (sizeof(T) == 8 ? 24576 : 20480);
-}
-template <int ORDER> constexpr int64_t team_min() { return ORDER >= 8 ? 49153 : 65537; }
-// Above this the FP64 walk goes back to one warp per group, whose 16 groups per
-// SM keep the FP64 pipe fuller (theta 0.4, Hernquist, wide / one warp, us):
-//   monopole 131,072: 1504 / 1645  190,000: 2184 / 2196  262,144: 3075 / 2876
-//   quad     190,000: 3296 / 3566  262,144: 4579 / 4711  2^20 (theta 0.5): 11697 / 10338
-//   octupole 131,072: 5220 / 5859  190,000: 7756 / 7832  262,144: 10914 / 10536
-template <int ORDER> constexpr int64_t wide64_max() { return ORDER == 4 ? 262144 : 196608; }
+// Which walk a launch takes (pipeline 1).  Few groups leave most of the chip idle,
+// so the more warps share a group the better; with more groups than a kernel has
+// producers (296 with 7 consumers a block, 592 with 3, 1,776 in teams, 2,368 one-warp
+// walks) the shared ones fall behind.  Where the lines lie depends on how long a
+// group's walk is: the walk of a small system is a pass or two, over before its
+// consumers gain anything.  So the choice goes by the number of groups, each
+// weighed by the length of its walk against the longest (about the square root of
+// the system's bodies, launch time taken off), and by the size of the largest system.
+// Walk times in us, 7 consumers / 3 consumers / teams / one warp a group (theta 0.5,
+// Plummer; g: ceil(n_s / group size) summed over the systems):
+//  FP32 quadrupole, one system    16,384 (g 256): 157 / 182 / 359 / -
+//                  20,480 (320): 196 / 204 / 404 / -   65,536 (1,024): 582 / 459 / 510 / -
+//                  100,003 (1,563): 876 / 654 / 549 / -
+//     monopole 20,480: 182 / 162 / 268   65,536: 526 / 354 / 326   octupole 32,768:
+//     450 / 497 / 635   65,536: 942 / 975 / 810
+//  FP32, groups of 32   6,000 (g 188): 88 / 100 / 153   20,000 (625): 247 / 173 / 240
+//                       40,000 (1,250): 481 / 317 / 285   65,000 (2,032): 810 / 506 / 385
+//     octupole 6,000: 104 / 126 / 200   20,000: 296 / 220 / 333   40,000: 599 / 465 / 500
+//              65,000: 1,023 / 753 / 754
+//  FP32, batches   4,000 systems of 10: 68 / 43 / 28 / 25   600 of 64: 35 / 28 / 27 / 29
+//     75 of 100 (g 150): 25 / 26 / 31 / 32   300 of 100 (600): 39 / 32 / 32 / 35
+//     37 of 500 (296): 55 / 43 / 63 / 73   75 of 500 (600): 90 / 71 / 64 / 75
+//     37 of 1,000 (592): 114 / 90 / 100 / -   62 of 1,000 (992): 178 / 140 / 103 / -
+//     15 of 4,000 (945): 276 / 217 / 244 / -   31 of 4,000 (1,953): 512 / 404 / 333 / -
+//     octupole, 75 of 100: 25 / 27 / 28   300 of 100: 41 / 33 / 28
+//  FP64 quadrupole, batches   300 of 10: 23 / 21 / - / 21   2,000 of 30: 62 / 43 / - / 28
+//     75 of 100: 27 / 29 / - / 41   500 of 100 (g 1,000): 58 / 43 / - / 48
+//     1,000 of 100 (2,000): 92 / 66 / - / 50   250 of 200 (1,000): 111 / 87 / - / 71
+//     1,000 of 200 (4,000): 400 / 330 / - / 158   62 of 1,000 (992): 235 / 196 / - / 238
+//     125 of 1,000 (2,000): 426 / 365 / - / 268   31 of 4,000 (1,953): 675 / 620 / - / 644
+//     63 of 4,000 (3,969): 1,301 / 1,169 / - / 1,035
+//  FP64, one system (theta 0.4 and 0.6, Hernquist and uniform sphere, 3 consumers over
+//     one warp a group, means of the four): quadrupole 131,072 0.85, 230,000 0.95,
+//     300,000 0.97, 350,000 1.03, 524,288 1.06; monopole 131,072 0.94, 196,608 1.16;
+//     octupole (7 consumers) 131,072 0.88, 196,608 1.04.
+//  Ranges of a 2^20-body system's groups, FP32 quadrupole   200: 251 / 311 / 653
+//     800: 489 / 387 / 666; FP64 quadrupole of 2^19   2,000: 1,473 / 1,408 / - / 1,766
+//     4,000: 2,761 / 2,572 / - / 2,744
+enum class Walk { kOneWarp, kTeams, kWide3, kWide7 };
+constexpr int64_t kLongWalks = 2048;  // bodies from which a system's walks are long
 
+template <typename T, int ORDER, int MAXTPL>
+static Walk choose_walk(const WalkArgs &a) {
+  if (!a.pipeline) return Walk::kOneWarp;
+  double g = a.walk_groups;
+  if (a.g_end >= 0) g = fmin(g, (double)(a.g_end - a.g_begin));
+  const double root = sqrt((double)a.largest);
+  const bool lone = a.largest >= kLongWalks;
+  double seven = 200.0, three;  // the most weighed groups of each
+  if constexpr (sizeof(T) == 8) {
+    const double most = ORDER >= 8 ? 2900.0 : (ORDER >= 4 ? 5000.0 : 2400.0);
+    three = a.largest <= kWarp ? 400.0 : fmin(fmax(40.0 * root, 800.0), most);
+    if (lone) seven = ORDER >= 8 ? three : 384.0;
+  } else if constexpr (ORDER >= 8) {
+    three = lone ? (MAXTPL == 2 ? 768.0 : 1400.0) : 400.0;
+    if (lone) seven = MAXTPL == 2 ? 768.0 : 400.0;
+  } else {
+    three = fmin(fmax(20.0 * root, 512.0), 1024.0);
+    if (lone) seven = 320.0;
+  }
+  if (g <= seven) return Walk::kWide7;
+  if (g <= three) return Walk::kWide3;
+  return sizeof(T) == 4 ? Walk::kTeams : Walk::kOneWarp;
+}
 
 template <typename T, int ORDER, int MAXTPL, bool SOFT>
 static void launch_group_walk(const WalkArgs &a, cudaStream_t s) {
-  if (a.pipeline && (sizeof(T) == 4 || a.n <= wide64_max<ORDER>())) {
-    if constexpr (sizeof(T) == 4) {
-      if (a.n >= team_min<ORDER>() && launch_team_walk<ORDER, MAXTPL, SOFT>(a, s)) return;
+  Walk kind = choose_walk<T, ORDER, MAXTPL>(a);
+  if constexpr (sizeof(T) == 4) {
+    if (kind == Walk::kTeams) {
+      if (launch_team_walk<ORDER, MAXTPL, SOFT>(a, s)) return;
+      kind = Walk::kWide3;
     }
-    if constexpr (ORDER < 8) {
-      if (a.n > seven_max<T, ORDER>()) {
-        launch_wide_walk<T, ORDER, MAXTPL, SOFT, 3>(a, s);
-        return;
-      }
-    }
-    launch_wide_walk<T, ORDER, MAXTPL, SOFT, 7>(a, s);
-    return;
   }
+  if (kind == Walk::kWide7) return launch_wide_walk<T, ORDER, MAXTPL, SOFT, 7>(a, s);
+  if (kind == Walk::kWide3) return launch_wide_walk<T, ORDER, MAXTPL, SOFT, 3>(a, s);
   static int per_sm[64] = {};
   const int per = resident_blocks(per_sm, group_walk_kernel<T, ORDER, MAXTPL, SOFT>, kWarp, 0);
   const int64_t blocks = bh_min64(a.slots, (int64_t)sm_count() * per);  // one stack per block
@@ -1821,6 +1858,8 @@ static WalkArgs make_args(int64_t n, const WalkParams &p, Buffers &b, double *ou
   a.mac = p.mac;
   a.g_begin = p.g_begin; a.g_end = p.g_end;
   a.pipeline = p.pipeline;
+  a.largest = b.largest;
+  a.walk_groups = b.walk_groups[p.group_size > 32 ? 1 : 0];
   return a;
 }
 
