@@ -33,26 +33,7 @@ constexpr int kDirSplits = 8;  // CTAs of a cluster (the portable limit), one so
 constexpr int kDirLanes = 64;  // threads of a group, one target each
 constexpr int kDirSubs = 4;    // groups of a CTA
 constexpr int kDirThreads = kDirLanes * kDirSubs;
-
-// One target's sum in the reference's own operations, for a result that did
-// not come out finite: coincident unsoftened bodies and squared distances
-// beyond the range of mass_over_r3 give what these operations give.
-__device__ __noinline__ void direct_plain(const double *__restrict__ m, const double *__restrict__ x,
-                                          const double *__restrict__ y,
-                                          const double *__restrict__ z, int64_t n, int64_t a,
-                                          double gm, double eps2, double f[3]) {
-  const double xa = x[a], ya = y[a], za = z[a];
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int64_t j = 0; j < n; ++j) {
-    if (j == a) continue;
-    const double dx = x[j] - xa, dy = y[j] - ya, dz = z[j] - za;
-    const double dist2 = dx * dx + dy * dy + dz * dz + eps2;
-    const double dist = sqrt(dist2);
-    const double w = gm * m[j] / (dist * dist2);
-    fx = fx + w * dx; fy = fy + w * dy; fz = fz + w * dz;
-  }
-  f[0] = fx; f[1] = fy; f[2] = fz;
-}
+static_assert(kDirLanes == 2 * kWarp, "two warps of targets");
 
 // SELF: the target may be among the sources of this tile
 template <bool SELF>
@@ -70,6 +51,82 @@ __device__ __forceinline__ void direct_tile(const double4 *tile, int cnt, int64_
   }
 }
 
+// Component q of target `lane`: the partial sums of the groups, slice by slice.
+__device__ __forceinline__ double cluster_sum(const cg::cluster_group &cluster, double *part, int q,
+                                              int lane) {
+  double f = 0.0;
+  for (int r = 0; r < kDirSplits; ++r) {
+    const double *p = cluster.map_shared_rank(part, r);
+    for (int g = 0; g < kDirSubs; ++g) f += p[(g * 3 + q) * kDirLanes + lane];
+  }
+  return f;
+}
+
+// What a thread of the cluster works on: target a (entry k of the output) and the
+// sources [s0, s1).
+struct DirSlot {
+  int64_t k, a, s0, s1;
+  bool bad;  // invalid target index: NaN result
+};
+__device__ __forceinline__ DirSlot direct_slot(int rank, int64_t n, const int64_t *targets, int64_t nt) {
+  DirSlot d;
+  d.k = (int64_t)(blockIdx.x / kDirSplits) * kDirLanes + threadIdx.x % kDirLanes;
+  d.a = d.k < nt ? (targets ? targets[d.k] : d.k) : 0;
+  d.bad = d.a < 0 || d.a >= n;
+  if (d.bad) d.a = 0;
+  d.s0 = n * rank / kDirSplits;
+  d.s1 = n * (rank + 1) / kDirSplits;
+  return d;
+}
+
+// Sums that did not come out finite, made again with the reference's own
+// operations by the whole cluster: coincident unsoftened bodies, non-finite inputs
+// and squared distances beyond the range of mass_over_r3 give what these operations
+// give.  `redo` has the targets of the thread's warp.  Not inlined and not unrolled:
+// with this sum in its body the kernel took 66 registers, which leaves 3 blocks per
+// SM (16,384 bodies 0.354 ms), or spills at 64 (0.322).  One NaN among 16,384 bodies, so that every sum
+// is made again: 1.0 ms, against 17.8 by the first warps of one CTA; a coincident pair
+// 0.34 against 4.4.
+__device__ __noinline__ void direct_again(const double *__restrict__ m, const double *__restrict__ x,
+                                          const double *__restrict__ y,
+                                          const double *__restrict__ z, int64_t n,
+                                          const int64_t *__restrict__ targets, int64_t nt, double G,
+                                          double eps2, int out_kind, double *__restrict__ out,
+                                          double4 *tile, double *part, unsigned redo) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int sub = threadIdx.x / kDirLanes, lane = threadIdx.x % kDirLanes;
+  const DirSlot d = direct_slot(rank, n, targets, nt);
+  const double gm = G * (out_kind == 1 ? 1.0 : m[d.a]);
+  const double xa = x[d.a], ya = y[d.a], za = z[d.a];
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  for (int64_t src = d.s0; src < d.s1; src += kDirThreads) {
+    const int64_t j = src + threadIdx.x;
+    __syncthreads();
+    if (j < d.s1) tile[threadIdx.x] = make_double4(x[j], y[j], z[j], m[j]);
+    __syncthreads();
+    const int64_t first = src + sub * kDirLanes;  // this group's part of the tile
+    const int cnt = (int)(redo && first < d.s1 ? bh_min64(kDirLanes, d.s1 - first) : 0);
+#pragma unroll 1
+    for (int i = 0; i < cnt; ++i) {
+      if (first + i == d.a) continue;
+      const double4 s = tile[sub * kDirLanes + i];
+      const double dx = s.x - xa, dy = s.y - ya, dz = s.z - za;
+      const double dist2 = dx * dx + dy * dy + dz * dz + eps2;
+      const double dist = sqrt(dist2);
+      const double w = gm * s.w / (dist * dist2);
+      fx = fx + w * dx; fy = fy + w * dy; fz = fz + w * dz;
+    }
+  }
+  part[(sub * 3 + 0) * kDirLanes + lane] = fx;
+  part[(sub * 3 + 1) * kDirLanes + lane] = fy;
+  part[(sub * 3 + 2) * kDirLanes + lane] = fz;
+  cluster.sync();
+  if (rank == 0 && sub == 0 && (redo >> (lane % kWarp) & 1u))
+    for (int q = 0; q < 3; ++q) out[q * nt + d.k] = cluster_sum(cluster, part, q, lane);
+  cluster.sync();
+}
+
 __global__ void __launch_bounds__(kDirThreads)
 direct_kernel(const double *__restrict__ m, const double *__restrict__ x,
               const double *__restrict__ y, const double *__restrict__ z, int64_t n,
@@ -77,16 +134,15 @@ direct_kernel(const double *__restrict__ m, const double *__restrict__ x,
               int out_kind, double *__restrict__ out) {
   __shared__ double4 tile[kDirThreads];
   __shared__ double part[kDirSubs][3][kDirLanes];
+  __shared__ unsigned again[kDirLanes / kWarp];  // targets whose sum is not finite
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int sub = threadIdx.x / kDirLanes, lane = threadIdx.x % kDirLanes;
-  const int64_t k = (int64_t)(blockIdx.x / kDirSplits) * kDirLanes + lane;
-  int64_t a = k < nt ? (targets ? targets[k] : k) : 0;
-  const bool bad = a < 0 || a >= n;  // invalid target index: NaN result
-  if (bad) a = 0;
+  const DirSlot d = direct_slot(rank, n, targets, nt);
+  if (threadIdx.x < kDirLanes / kWarp) again[threadIdx.x] = 0;
+  const int64_t a = d.a, s0 = d.s0, s1 = d.s1;
   const double xa = x[a], ya = y[a], za = z[a];
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  const int64_t s0 = n * rank / kDirSplits, s1 = n * (rank + 1) / kDirSplits;
   for (int64_t src = s0; src < s1; src += kDirThreads) {
     const int64_t j = src + threadIdx.x;
     __syncthreads();
@@ -102,21 +158,22 @@ direct_kernel(const double *__restrict__ m, const double *__restrict__ x,
   }
   part[sub][0][lane] = fx; part[sub][1][lane] = fy; part[sub][2][lane] = fz;
   cluster.sync();
-  if (rank == 0 && sub == 0 && k < nt) {
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int r = 0; r < kDirSplits; ++r) {
-      const double *p = cluster.map_shared_rank(&part[0][0][0], r);
-      for (int g = 0; g < kDirSubs; ++g)
-        for (int q = 0; q < 3; ++q) f[q] += p[(g * 3 + q) * kDirLanes + lane];
-    }
-    const double gm = G * (out_kind == 1 ? 1.0 : m[a]);
-    for (int q = 0; q < 3; ++q) f[q] = gm * f[q];
-    if (!(isfinite(f[0]) && isfinite(f[1]) && isfinite(f[2])))
-      direct_plain(m, x, y, z, n, a, gm, eps2, f);
-    if (bad) f[0] = f[1] = f[2] = nan("");
-    out[k] = f[0]; out[nt + k] = f[1]; out[2 * nt + k] = f[2];
+  if (rank == 0 && sub == 0) {
+    const double gm = G * (out_kind == 1 ? 1.0 : m[d.a]);
+    double f[3];
+    for (int q = 0; q < 3; ++q) f[q] = gm * cluster_sum(cluster, &part[0][0][0], q, lane);
+    const bool finite = isfinite(f[0]) && isfinite(f[1]) && isfinite(f[2]);
+    const unsigned redo = __ballot_sync(0xffffffffu, d.k < nt && !d.bad && !finite);
+    if (redo && lane % kWarp < kDirSplits)  // every CTA of the cluster gets the word
+      cluster.map_shared_rank(again, lane % kWarp)[lane / kWarp] = redo;
+    if (d.bad) f[0] = f[1] = f[2] = nan("");
+    if (d.k < nt)
+      for (int q = 0; q < 3; ++q) out[q * nt + d.k] = f[q];
   }
-  cluster.sync();  // the other CTAs' shared memory stays until rank 0 has read it
+  cluster.sync();  // the words are set, and rank 0 has read the other CTAs' shared memory
+  if ((again[0] | again[1]) != 0)  // the same words in every CTA
+    direct_again(m, x, y, z, n, targets, nt, G, eps2, out_kind, out, tile, &part[0][0][0],
+                 again[lane / kWarp]);
 }
 
 constexpr int kProbeIters = 4096;

@@ -55,3 +55,64 @@ def test_direct_sum_special_values():
     near = np.array([[0.0, 0.0, 0.0], [1e-120, 0.0, 0.0]])
     f = _direct(m[:2], near)
     assert f[0, 0] == np.inf and f[1, 0] == -np.inf
+
+
+@pytest.mark.parametrize("n", [65, 130, 1025])
+def test_direct_sum_again_beside_finite_targets(n):
+    """Sums made again in the reference's operations -- a light body so close to a
+    heavy one that m / r^3 overflows and G m_a m / r^3 does not, a coincident pair,
+    one NaN -- in the first, a middle and the last tile of targets, beside targets
+    that keep their first sum.  r^3 is subnormal there: 1e-6 of its value at least."""
+    rng = np.random.default_rng(n)
+    m, q = rng.uniform(0.5, 1.5, n), rng.normal(size=(n, 3)) + 5.0
+    clean = _direct(m, q)
+    for a, b in ((0, n - 1), (n // 2, 3), (n - 1, n // 2)):
+        m2, q2 = m.copy(), q.copy()
+        q2[a], q2[b], m2[a] = 0.0, 0.0, 1e-100
+        q2[b, 0] = 1e-105
+        f = _direct(m2, q2)
+        t = m2[a] * m2[b] / (1e-105 * (1e-105 * 1e-105))
+        assert abs(f[a, 0] / (t * 1e-105) - 1.0) < 1e-6 and np.isfinite(f[a]).all()
+        q2[b] = q2[a]  # coincident, unsoftened
+        f = _direct(m2, q2)
+        rest = np.delete(np.arange(n), [a, b])
+        assert np.isnan(f[[a, b]]).all() and np.isfinite(f[rest]).all()
+        tg = np.array([rest[0], a, rest[-1], b, -1])
+        g = _direct(m2, q2, tg)
+        assert np.array_equal(g[[0, 2]], f[[rest[0], rest[-1]]]) and np.isnan(g[[1, 3, 4]]).all()
+        q2[b] = q[b]
+        q2[a, 1] = np.nan
+        f = _direct(m2, q2)
+        assert np.isnan(f[:, 1]).all()
+    assert np.array_equal(clean, _direct(m, q))
+
+
+def test_direct_sum_of_degraded_inputs_stays_parallel():
+    """Making sums again costs what all pairs in the reference's operations cost
+    (about 3 times the clean call where all of them are made again, 52 times by two
+    warps of a cluster), or one tile's share of it."""
+    import torch
+
+    from hierarquicos_b200.system import direct_targets
+
+    rng = np.random.default_rng(1)
+    n = 16384
+    q = rng.normal(size=(3, n))
+    pair, nan = q.copy(), q.copy()
+    pair[:, 1] = pair[:, 0]
+    nan[0, n // 2] = np.nan
+    m = torch.full((n,), 1.0 / n, dtype=torch.float64, device="cuda")
+    best = []
+    for p in (q, pair, nan):
+        args = [m] + [torch.from_numpy(np.ascontiguousarray(r)).cuda() for r in p]
+        t = []
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            direct_targets(*args)
+            a.record()
+            direct_targets(*args)
+            b.record()
+            torch.cuda.synchronize()
+            t.append(a.elapsed_time(b))
+        best.append(min(t))
+    assert best[1] <= 3.0 * best[0] and best[2] <= 25.0 * best[0], best
