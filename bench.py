@@ -202,7 +202,7 @@ def launches_per_evaluation(n, nsys=1, L=21):
     """Our kernel launches in one build + walk of nsys equal systems (the
     pipeline's launch sequence: 40 for one system of 2^20 bodies)."""
     keys = 3                                           # reduce, finalize, keys
-    if n * n / nsys <= (1.44e8 if nsys == 1 else 2.5e8):
+    if n * n / nsys <= (1.44e8 if nsys == 1 else min(3e7 + 4500 * n, 7e8)):
         sort = 1                                       # places by counting
     else:                                              # digit scan, passes, gather
         spass = math.ceil(math.log2(nsys) / 8) if nsys > 1 else 0

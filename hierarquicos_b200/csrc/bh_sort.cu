@@ -18,6 +18,8 @@
 // equal digits land on consecutive addresses.  A block only waits for tiles
 // claimed before its own, by blocks that are already running; every wait is
 // bounded and a wait that gives up raises an error flag instead of hanging.
+#include <math.h>
+
 #include "bh_internal.cuh"
 #include "bh_lookback.cuh"
 
@@ -32,12 +34,19 @@ constexpr int kSmallItems = kSortTileSmall / 256;  // and of a small sort's
 constexpr int kTile = kSortThreads * kItems;  // 4096 keys per block (large sorts)
 constexpr int kRadix = 256;
 
-// Sum over the systems of n_s^2 up to which a batch is sorted by counting; above
-// it the comparisons cost more than the radix passes.  Whole builds, us, counting
-// / radix: one system of 1,024 bodies 69 / 101, 8,192 110 / 127, 12,000 128 / 131,
-// 16,384 202 / 138; batches (whose radix sort has passes over the system too) of
-// 1.4e8 in 48 systems 159 / 233, in 16 systems 179 / 167, 6.7e8 293 / 269.
-constexpr double kRankPairsOne = 1.44e8, kRankPairsBatch = 2.5e8;
+// Sum over the systems of n_s^2 up to which bodies are sorted by counting; above
+// it the comparisons cost more than the radix passes, which in a batch grow with the
+// bodies (more tiles, and passes over the system too).  Whole builds, us, counting /
+// radix (Plummer; uniform spheres cross at the same sizes):
+//   one system   10,000 (1e8) 151 / 159   12,000 (1.4e8) 156 / 160   14,142 (2e8) 194 / 162
+//   2 of 7,071 (1e8) 153 / 168   2 of 8,485 (1.4e8) 180 / 173   2 of 11,180 (2.5e8) 261 / 182
+//   4 of 5,000 (1e8) 171 / 175   4 of 6,000 (1.4e8) 197 / 182
+//   8 of 4,242 (1.4e8) 208 / 211   8 of 5,000 (2e8) 219 / 216   8 of 6,614 (3.5e8) 235 / 224
+//   16 of 4,677 (3.5e8) 227 / 253   16 of 5,590 (5e8) 254 / 256   16 of 6,614 (7e8) 294 / 260
+//   32 of 3,952 (5e8) 255 / 268   32 of 4,677 (7e8) 307 / 277
+//   128 of 2,338 (7e8) 348 / 388   512 of 1,169 (7e8) 451 / 499
+constexpr double kRankPairsOne = 1.44e8;
+inline double rank_pairs_batch(int64_t n) { return fmin(3e7 + 4500.0 * (double)n, 7e8); }
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
@@ -445,7 +454,7 @@ int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, in
 
 SortPlan sort_plan(int64_t n, int L, const Buffers &b) {
   SortPlan p;
-  p.by_rank = b.sort_pairs <= (b.nsys > 1 ? kRankPairsBatch : kRankPairsOne);
+  p.by_rank = b.sort_pairs <= (b.nsys > 1 ? rank_pairs_batch(n) : kRankPairsOne);
   const int bits = 3 * (L == 0 ? kMaxDepth : L);
   p.kpass = (bits + 7) / 8;
   p.spass = 0;

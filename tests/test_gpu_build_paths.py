@@ -147,3 +147,26 @@ def test_batch_radix_places(sizes):
         assert np.array_equal(keys[a:e], k1) and np.array_equal(perm[a:e] - a, p1), s
     b.close()
     lone.close()
+
+
+@pytest.mark.parametrize("sizes", [[6700] * 2, [6760] * 2, [5750] * 4, [5840] * 4, [4850] * 16,
+                                   [4920] * 16, [2330] * 128, [2345] * 128])
+def test_batches_on_both_sides_of_the_sorts_line(sizes):
+    """Just below and above the sum of n_s^2 up to which a batch is sorted by
+    counting: the same places as lone builds (counting up to 12,000 bodies)."""
+    from hierarquicos_b200.system import BHSystem, offsets_of
+
+    m, q = _cloud(sum(sizes), 12)
+    off = offsets_of(sizes)
+    b, lone = BHSystem(), BHSystem()
+    b.build_batch(m, *xyz(q), off)
+    b.sync()
+    keys, perm = b.keys()
+    for s in sorted({0, 1, len(sizes) - 1}):
+        a, e = int(off[s]), int(off[s + 1])
+        lone.build(m[a:e], *xyz(q[a:e]))
+        lone.sync()
+        k1, p1 = lone.keys()
+        assert np.array_equal(keys[a:e], k1) and np.array_equal(perm[a:e] - a, p1), s
+    b.close()
+    lone.close()
