@@ -170,3 +170,97 @@ def test_batches_on_both_sides_of_the_sorts_line(sizes):
         assert np.array_equal(keys[a:e], k1) and np.array_equal(perm[a:e] - a, p1), s
     b.close()
     lone.close()
+
+
+def _chain(n):
+    """Bodies that halve their distance to a corner, and some exact duplicates."""
+    rng = np.random.default_rng(4)
+    q = rng.uniform(0.5, 1.0, size=(n, 3)) * 2.0 ** -rng.integers(0, 20, size=(n, 1))
+    q = np.concatenate([q, q[:300]])
+    return rng.uniform(0.5, 1.5, len(q)) / len(q), q
+
+
+def _all_moments(m, q, nodes, perm, order):
+    """Every node's mass, centre, second and third moments from its bodies, level by
+    level (the nodes of a level hold disjoint ranges).  The second and third moments
+    are taken about the node's own centre; a child's centre is off by a few roundings
+    of |r| a level, at most 21 levels, and the translation takes its dipole for zero:
+    3 * 40 u |r| / size, with |r| / size below 2^20 (below that the moments are
+    measured against |r| 2^-20): 1.4e-8."""
+    ms, qs = m[perm], q[perm]
+    n = len(ms)
+    for level in np.unique(nodes["meta"][:, 2]):
+        j = np.flatnonzero(nodes["meta"][:, 2] == level)
+        f, c = nodes["meta"][j, 0].astype(int), nodes["meta"][j, 1].astype(int)
+        ends = np.stack([f, f + c], 1).ravel()
+
+        def total(v):
+            return np.add.reduceat(np.append(v, 0.0), np.minimum(ends, n))[::2]
+
+        body = np.repeat(np.arange(len(j)), c)
+        at = np.concatenate([np.arange(a, b) for a, b in zip(f, f + c)])
+        tol = 4 * (c + 64) * 2.0 ** -53
+        mass = total(ms)
+        assert (np.abs(nodes["com"][j, 3] - mass) <= tol * mass).all(), level
+        com = nodes["com"][j, :3]
+        for k in range(3):
+            ref, size = total(ms * qs[:, k]) / mass, total(np.abs(ms * qs[:, k])) / mass
+            assert (np.abs(com[:, k] - ref) <= tol * size + 1e-300).all(), level
+        if order < 4:
+            continue
+        d = np.zeros((n, 3))
+        d[at] = qs[at] - com[body]
+        r = np.zeros(len(j))
+        np.maximum.at(r, body, np.abs(d[at]).max(1))
+        size = r + np.abs(com).max(1) * 2.0 ** -20
+        for k, (a, b) in enumerate(((0, 0), (1, 1), (2, 2), (0, 1), (0, 2), (1, 2))):
+            got = nodes["quad"][j, k]
+            assert (np.abs(got - total(ms * d[:, a] * d[:, b])) <= 2e-8 * mass * size ** 2).all(), (level, k)
+        if order < 8:
+            continue
+        third = ((0, 0, 0), (0, 1, 1), (0, 2, 2), (0, 0, 1), (1, 1, 1), (1, 2, 2), (0, 0, 2), (1, 1, 2),
+                 (2, 2, 2), (0, 1, 2))
+        for k, (a, b, e) in enumerate(third):
+            got = nodes["oct"][j, k]
+            assert (np.abs(got - total(ms * d[:, a] * d[:, b] * d[:, e])) <= 2e-8 * mass * size ** 3).all(), (level, k)
+
+
+@pytest.mark.parametrize("order", [1, 4, 8])
+@pytest.mark.parametrize("n", [257, 32768, 32769, 65536, 65537, -40000, -65236, -70000])
+def test_moments_of_every_stage(n, order):
+    """One chunk and one list, both list stages, and level by level; n < 0: the
+    nested chain, whose nodes span chunks on every level (65,536 bodies the most
+    that go in stages)."""
+    from hierarquicos_b200.system import BHSystem
+
+    m, q = _cloud(n, 3) if n > 0 else _chain(-n)
+    s = BHSystem()
+    s.build(m, *xyz(q), order=order)
+    s.sync()
+    _all_moments(m, q, s.nodes(), s.keys()[1], order)
+    s.close()
+
+
+@pytest.mark.parametrize("order", [4, 8])
+def test_staged_and_levelled_moments_are_the_same(order):
+    """Systems of a batch of more than 65,536 bodies go level by level, alone in
+    stages: the same centres, moments and forces, bit for bit."""
+    from hierarquicos_b200.system import BHSystem, offsets_of
+
+    parts = [_cloud(40000, 1), _chain(20000), _cloud(300, 2), _cloud(33000, 3)]
+    m, q = np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
+    off = offsets_of([len(p[0]) for p in parts])
+    b, lone = BHSystem(), BHSystem()
+    f = b.forces_batch(m, *xyz(q), off, order=order, theta=0.6, eps=0.01).cpu().numpy()
+    all_nodes = b.nodes()
+    for s in range(len(parts)):
+        a, e = int(off[s]), int(off[s + 1])
+        g = lone.forces(m[a:e], *xyz(q[a:e]), order=order, theta=0.6, eps=0.01).cpu().numpy()
+        nodes = lone.nodes()
+        first = all_nodes["meta"][:, 0]
+        j = np.flatnonzero((first >= a) & (first < e))
+        for name in ("com", "quad", "oct")[:2 if order < 8 else 3]:
+            assert np.array_equal(all_nodes[name][j], nodes[name]), (s, name)
+        assert np.array_equal(f[3 * a:3 * e], g), s
+    b.close()
+    lone.close()
