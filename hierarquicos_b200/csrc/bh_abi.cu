@@ -331,7 +331,7 @@ void enqueue_build(bh_system *s, int keys_from_scalars, cudaStream_t st) {
   bh::launch_sort(s->m, s->x, s->y, s->z, n, L, b, st);
   if (L == 0) bh::launch_auto_depth(n, b, st);
   bh::launch_build_tree(n, b, st);
-  bh::launch_upward(n, L, p.order, b, st);
+  bh::launch_upward(n, p.order, b, st);
   bh::launch_groups(n, p.group_size, p.group_span > 0 ? p.group_span : 2 * p.group_size, b, st);
 }
 

@@ -685,10 +685,9 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
       uint64_t *st = d.gen_status + (int64_t)g * 2 * max_tiles;
       // the resident blocks (they claim tiles until none is left); most of the
       // generations are small or empty, so the launch itself counts
-      launch_pdl(
-          dual_gen_kernel, 148 * kGenBlocksPerSm, kGenThreads, 0, s, e, fi, cnt + (g & 1), fcap, fo,
-          cnt + ((g + 1) & 1), fcap, d.mut, cnt + 2 + (g & 1), cnt + 2 + ((g + 1) & 1), d.mut_cap, p.theta2, cnt + 4, st, st + max_tiles,
-          d.gen_tiles + g, &b.sc->err);
+      launch_pdl(dual_gen_kernel, 148 * kGenBlocksPerSm, kGenThreads, 0, s, e, fi, cnt + (g & 1), fcap,
+                 fo, cnt + ((g + 1) & 1), fcap, d.mut, cnt + 2 + (g & 1), cnt + 2 + ((g + 1) & 1),
+                 d.mut_cap, p.theta2, cnt + 4, st, st + max_tiles, d.gen_tiles + g, &b.sc->err);
       if (g + 1 != kFirstGenerations && g + 1 != kGenerations) continue;
       if (cudaMemcpyAsync(h, d.counters, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                           s) != cudaSuccess ||
@@ -728,7 +727,7 @@ int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, dou
                             &b.sc->err, s, d.cnt, ne) == 1)
       sources = d.vals + nh;
   }
-  exclusive_scan(d.cnt, d.beg, ne + 1, nullptr, nullptr, d.scan_tmp, &b.sc->err, s);
+  exclusive_scan(d.cnt, d.beg, ne + 1, d.scan_tmp, &b.sc->err, s);
   const int egrid = grid_for(ne * kEvalLanes, 128, 148 * 32);
   const double G = p.G, eps2 = p.eps2;
   if (p.order >= 8)

@@ -215,23 +215,21 @@ void launch_sort(const double *m, const double *x, const double *y, const double
 
 // stable LSD radix sort of 32-bit keys over bits [0, bits) when only the values
 // are wanted: the last pass writes no keys and nothing is copied back; returns
-// the buffer holding the sorted values (0: v0, 1: v1).  key_counts, if given, holds the number of keys
-// of every key value 0..n_key_values-1 (the digit counts then come from it
-// instead of from a pass over the keys).
+// the buffer holding the sorted values (0: v0, 1: v1).  key_counts holds the number
+// of keys of every key value 0..n_key_values-1; the digit counts come from it.
 int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n, int bits,
                         int32_t *hist, int *err, cudaStream_t s,
-                        const int32_t *key_counts = nullptr, int64_t n_key_values = 0);
+                        const int32_t *key_counts, int64_t n_key_values);
 // scratch of the scan, in int32 entries: a ticket and a 64-bit word per
-// 8192-value tile; scratch of the radix sort: digit counts of 8 passes x 256
-// digits, 8 tile counters, and a 64-bit word per (pass, 4096-key tile, digit)
+// 8192-value tile
 constexpr int64_t scan_tmp_entries(int64_t n) { return 2 * ((n + 8191) / 8192) + 4; }
 // scratch of the tree, group and upward passes of a build (layout: bh_tree.cu),
 // in int32 entries
 constexpr int64_t kTreeTile = 256, kGroupScanTile = 2048;
-constexpr int64_t upward_counter_entries(int64_t n) { return (n >> 15) + (n >> 22) + (n >> 29) + 4; }
+constexpr int64_t kUpwardCounters = 4;  // lists of the staged upward pass (bh_upward.cu)
 constexpr int64_t build_tmp_entries(int64_t n) {
   return 2 + kWarp + 2 * kWarp * ((n + kTreeTile - 1) / kTreeTile) +
-         2 * ((n + kGroupScanTile - 1) / kGroupScanTile) + upward_counter_entries(n);
+         2 * ((n + kGroupScanTile - 1) / kGroupScanTile) + kUpwardCounters;
 }
 // radix sort tiles: sorts of at most kSortSmallMax keys use small tiles (more
 // blocks in flight: a 2^14-body build 0.380 -> 0.350 ms), larger ones large
@@ -250,17 +248,15 @@ constexpr int64_t radix_hist_entries(int64_t n, int passes = kMaxSortPasses) {
   return passes * 256 + 12 + 2 * passes * 256 * radix_tiles(n);
 }
 
-// exclusive scan of n int32 values in one launch; total written to *total
-// and *total2 (device) when given; a look-back wait that gives up sets
-// kErrTimeout in *err
-void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n_dev,
-                    int32_t *total, int32_t *tmp, int *err, cudaStream_t s,
-                    int32_t *total2 = nullptr);
+// exclusive scan of n int32 values in one launch; a look-back wait that gives up
+// sets kErrTimeout in *err
+void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, int *err,
+                    cudaStream_t s);
 
 void launch_build_tree(int64_t n, Buffers &b, cudaStream_t s);
 // the upward pass's list counters (cleared with the rest of scan_tmp)
 int32_t *upward_counters(int64_t n, Buffers &b);
-void launch_upward(int64_t n, int L, int order, Buffers &b, cudaStream_t s);
+void launch_upward(int64_t n, int order, Buffers &b, cudaStream_t s);
 void launch_groups(int64_t n, int group_size, int group_span, Buffers &b, cudaStream_t s);
 
 // Runs the check of the pipelined walk's bounded mbarrier waits (one block
@@ -276,7 +272,7 @@ struct WalkParams {
   int leaf_cap;
   int count_stats;
   int mac;         // 0 box distance, 1 box distance or every member's own MAC
-  int pipeline = 0;  // FP32 walk: 0 one warp per group, 1 producer/consumer warps
+  int pipeline = 0;  // 0 one warp per group, 1 producer / consumer warps where they are faster
   int g_begin = 0, g_end = -1;  // target groups walked: [g_begin, g_end), g_end < 0 = all
   // The walk directly follows a build in the same stream or graph, which left the
   // group cursor at 0.  Only a call that queues both may say so: any other walk may
@@ -306,14 +302,15 @@ struct DehnenBuffers {
   int64_t pairs = 0;                      // mutual interactions of the last run
 };
 // Dehnen's method over the built batch into out (same layout as the walk).
-// Synchronises the stream once (to size the pair lists).  Returns 0, 1 out of
+// Synchronises the stream to size the pair lists: after 32 generations of the
+// traversal, after all 50 if pairs are left then, and so again after every attempt
+// whose lists were too short.  Returns 0, 1 out of
 // device memory, 2 CUDA error, 3 traversal did not close, 4 pair lists too
 // large.
 int run_dehnen(int64_t n, const WalkParams &p, Buffers &b, DehnenBuffers &d, double *out,
                cudaStream_t s);
 void free_dehnen(DehnenBuffers &d);
 
-// Returns the number of warp slots used (for stack sizing).
 void launch_walk(int64_t n, const WalkParams &p, Buffers &b, double *out, cudaStream_t s);
 void launch_reference_walk(int64_t n, const WalkParams &p, Buffers &b, double *out,
                            const int64_t *targets, int64_t ntargets, int64_t *counts,

@@ -109,17 +109,17 @@ reduce_partials(const double *__restrict__ m, const double *__restrict__ x,
     for (int q = 0; q < kRedBatch; ++q) {
       if (p0 + q * kRedThreads >= it.end) break;
       const double a = av[q], b = bv[q], c = cv[q], w = wv[q];
-    mn[0] = fmin(mn[0], a); mx[0] = fmax(mx[0], a);
-    mn[1] = fmin(mn[1], b); mx[1] = fmax(mx[1], b);
-    mn[2] = fmin(mn[2], c); mx[2] = fmax(mx[2], c);
-    sm = __dadd_rn(sm, w);
-    if (com_mode) {
-      sx = __fma_rn(w, a, sx); sy = __fma_rn(w, b, sy); sz = __fma_rn(w, c, sz);
-    } else {
-      sx = __dadd_rn(sx, __dmul_rn(w, a));
-      sy = __dadd_rn(sy, __dmul_rn(w, b));
-      sz = __dadd_rn(sz, __dmul_rn(w, c));
-    }
+      mn[0] = fmin(mn[0], a); mx[0] = fmax(mx[0], a);
+      mn[1] = fmin(mn[1], b); mx[1] = fmax(mx[1], b);
+      mn[2] = fmin(mn[2], c); mx[2] = fmax(mx[2], c);
+      sm = __dadd_rn(sm, w);
+      if (com_mode) {
+        sx = __fma_rn(w, a, sx); sy = __fma_rn(w, b, sy); sz = __fma_rn(w, c, sz);
+      } else {
+        sx = __dadd_rn(sx, __dmul_rn(w, a));
+        sy = __dadd_rn(sy, __dmul_rn(w, b));
+        sz = __dadd_rn(sz, __dmul_rn(w, c));
+      }
     }
   }
   int t = threadIdx.x;
@@ -459,10 +459,10 @@ static void run_keys(const double *m, const double *x, const double *y, const do
   }
   const bool odd = (plan.kpass + plan.spass) & 1;  // the passes end in k0, v0
   cudaMemsetAsync(b.hist, 0, plan.scratch * sizeof(int32_t), s);
-  launch_pdl(
-      keys_kernel<CHECK, true>, grid_for(n, 256, 148 * 8), 256, 0, s, m, x, y, z, n, depth, b.sys_of, b.ss, b.sc, odd ? b.k1 : b.k0, odd ? b.v1 : b.v0,
-      reinterpret_cast<double4 *>(b.cn_oct), plan.kpass, plan.spass,
-      reinterpret_cast<uint32_t *>(b.hist));
+  launch_pdl(keys_kernel<CHECK, true>, grid_for(n, 256, 148 * 8), 256, 0, s, m, x, y, z, n, depth,
+             b.sys_of, b.ss, b.sc, odd ? b.k1 : b.k0, odd ? b.v1 : b.v0,
+             reinterpret_cast<double4 *>(b.cn_oct), plan.kpass, plan.spass,
+             reinterpret_cast<uint32_t *>(b.hist));
 }
 
 void launch_keys(const double *m, const double *x, const double *y, const double *z, int64_t n,

@@ -136,8 +136,8 @@ struct PassSmem {
 // keys nobody reads).
 // 3 blocks per SM (80 registers, no spills; the compiler's own choice was 128
 // and 2 blocks): the 181 M-term sort of Dehnen's method 1 ms faster.
-// starts: first place of each of the pass's 256 digits.  SYS: the digit is the system's (of the body that the value names), not the
-// key's.
+// starts: first place of each of the pass's 256 digits.  SYS: the digit is the
+// system's (of the body that the value names), not the key's.
 template <typename K, int ITEMS, bool SYS>
 __global__ void __launch_bounds__(kSortThreads, 3)
 onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
@@ -228,8 +228,7 @@ onesweep_kernel(const K *__restrict__ kin, const int32_t *__restrict__ vin,
 // bounded and one that gives up raises kErrTimeout in *err.
 // tmp (int32 entries): [0] ticket, [1] unused, then one 64-bit word per tile.
 __global__ void __launch_bounds__(kScanThreads)
-scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n_max,
-                    const int32_t *n_dev, int32_t *tmp, int32_t *total_out, int32_t *total_out2,
+scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n, int32_t *tmp,
                     int *err) {
   __shared__ int ws[kScanThreads / kWarp];
   __shared__ int s_tile;
@@ -237,9 +236,6 @@ scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, i
   if (threadIdx.x == 0) s_tile = atomicAdd(tmp, 1);
   __syncthreads();
   const int t = s_tile;
-  const int64_t n = n_dev ? bh_min64(n_max, (int64_t)*n_dev) : n_max;
-  const int64_t ntiles = n > 0 ? (n + kScanChunk - 1) / kScanChunk : 1;
-  if ((int64_t)t >= ntiles) return;  // uniform across the block
   uint64_t *words = reinterpret_cast<uint64_t *>(tmp + 2);
   const int64_t base = (int64_t)t * kScanChunk + (int64_t)threadIdx.x * kScanItems;
   int vals[kScanItems];
@@ -253,13 +249,7 @@ scan_onepass_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, i
   int off = block_excl_scan(sum, ws, &tile_total);
   if (threadIdx.x < kWarp) {
     const int64_t excl = warp_lookback(words, t, tile_total, err);
-    if (threadIdx.x == 0) {
-      s_excl = excl;
-      if ((int64_t)t == ntiles - 1) {
-        if (total_out) *total_out = (int32_t)(excl + tile_total);
-        if (total_out2) *total_out2 = (int32_t)(excl + tile_total);
-      }
-    }
+    if (threadIdx.x == 0) s_excl = excl;
   }
   __syncthreads();
   int64_t o = s_excl + off;
@@ -383,8 +373,8 @@ void launch_pass(int64_t ntiles, const K *ki, const int32_t *vi, K *ko, int32_t 
                          smem);
     done[dev] = true;
   }
-  launch_pdl(
-      onesweep_kernel<K, ITEMS, SYS>, ntiles, kSortThreads, smem, s, ki, vi, ko, vo, n, shift, sys_of, counts, tiles, ctr, err);
+  launch_pdl(onesweep_kernel<K, ITEMS, SYS>, ntiles, kSortThreads, smem, s, ki, vi, ko, vo, n, shift,
+             sys_of, counts, tiles, ctr, err);
 }
 
 // scratch layout (int32 entries): digit counts [passes][256], tile counters
@@ -424,12 +414,12 @@ static_assert(kScanChunk == 8192 && kTile == kSortTileLarge && kRadix == 256 &&
                   kSortThreads * kSmallItems == kSortTileSmall && kMaxSortPasses <= 12,
               "scan_tmp_entries / radix_hist_entries in bh_internal.cuh assume these sizes");
 
-void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, const int32_t *n_dev,
-                    int32_t *total, int32_t *tmp, int *err, cudaStream_t s, int32_t *total2) {
+void exclusive_scan(const int32_t *in, int32_t *out, int64_t n, int32_t *tmp, int *err,
+                    cudaStream_t s) {
   int nb = (int)((n + kScanChunk - 1) / kScanChunk);
   if (nb < 1) nb = 1;
   cudaMemsetAsync(tmp, 0, (2 + 2 * (int64_t)nb) * sizeof(int32_t), s);
-  scan_onepass_kernel<<<nb, kScanThreads, 0, s>>>(in, out, n, n_dev, tmp, total, total2, err);
+  scan_onepass_kernel<<<nb, kScanThreads, 0, s>>>(in, out, n, tmp, err);
 }
 
 int radix_sort_values32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n, int bits,
@@ -467,8 +457,8 @@ void launch_sort(const double *m, const double *x, const double *y, const double
                  int L, Buffers &b, cudaStream_t s) {
   const SortPlan plan = sort_plan(n, L, b);
   if (plan.by_rank) {
-    launch_pdl(
-        rank_sort_kernel, (n + kRankBodies - 1) / kRankBodies, kRankWarps * kWarp, 0, s, b.k1, m, x, y, z, n, b.sys_of, b.ss, b.k0, b.v0, b.spos);
+    launch_pdl(rank_sort_kernel, (n + kRankBodies - 1) / kRankBodies, kRankWarps * kWarp, 0, s, b.k1, m,
+               x, y, z, n, b.sys_of, b.ss, b.k0, b.v0, b.spos);
     return;
   }
   const int passes = plan.kpass + plan.spass;
@@ -487,8 +477,8 @@ void launch_sort(const double *m, const double *x, const double *y, const double
     uint64_t *tk = ki; ki = ko; ko = tk;
     int32_t *tv = vi; vi = vo; vo = tv;
   }
-  launch_pdl(
-      gather_kernel, grid_for(n, 256, 148 * 16), 256, 0, s, reinterpret_cast<const double4 *>(b.cn_oct), b.v0, n, b.spos);
+  launch_pdl(gather_kernel, grid_for(n, 256, 148 * 16), 256, 0, s,
+             reinterpret_cast<const double4 *>(b.cn_oct), b.v0, n, b.spos);
 }
 
 }  // namespace bh

@@ -17,9 +17,9 @@
 // overlap.
 //
 // Systems of up to kChunkMax bodies, for which the 22 launches cost more than
-// their work, run in stages instead.  A node's range of bodies lies inside an
-// aligned chunk of 2^8, 2^15, 2^22 or 2^29 bodies (or none): the stage of the
-// smallest one computes it, so all its children are done by earlier stages or by
+// their work, run in three stages instead.  A node's range of bodies lies inside an
+// aligned chunk of 2^8 or 2^15 bodies or spans those: the stage of the smallest one
+// that holds it computes it, so all its children are done by earlier stages or by
 // the same block.  Stage 1 takes one block per 256 bodies, a thread per binary
 // node, with the chunk's bodies and results in shared memory; nodes that span its
 // chunks go on lists (one per chunk of the next stage that holds them), and the
@@ -319,7 +319,7 @@ struct UpArgs {
   double4 *com;
   double *quad, *oct;
   float4 *fq, *fo;
-  int32_t *list1, *list2, *count;  // lists of stage 2 and of the later stages
+  int32_t *list1, *list2, *count;  // lists of stages 2 and 3
   int *err;
   int64_t n;
 };
@@ -354,22 +354,21 @@ __device__ __forceinline__ void store_node(const UpArgs &a, int64_t j, const Mom
 constexpr int kChunkBits = 8, kChunk = 1 << kChunkBits, kStageBits = 7;
 constexpr int kListCap = ((1 << kStageBits) - 1) * (kMaxDepth + 1);  // nodes of one list
 constexpr int kUpThreads = 256;
+constexpr int64_t kChunkMax = 65536;  // the most bodies that go in stages
+static_assert(kChunkMax <= (int64_t)1 << (kChunkBits + 2 * kStageBits), "three stages hold every node");
+static_assert((kChunkMax >> (kChunkBits + kStageBits)) + 2 <= kUpwardCounters, "a counter per list");
 
-// list of a chunk of stage `stage` >= 2 (chunks of 2^(8 + 7 (stage - 1)) bodies):
-// stage 2 has list1 to itself, the later ones follow one another in list2.
-// Lists are kListCap entries apart; a last, partial chunk holds fewer nodes than
-// bodies, so the arrays of n entries hold them all.
+// list of a chunk of stage 2 (2^15 bodies) or 3 (all of them).  Stage 2's lists are
+// kListCap entries apart; a last, partial chunk holds fewer nodes than bodies, so the
+// arrays of n entries hold them all.
 __device__ __forceinline__ int32_t *up_list(const UpArgs &a, int stage, int64_t chunk,
                                             int32_t *&count) {
-  count = a.count;
-  int32_t *l = stage == 2 ? a.list1 : a.list2;
-  for (int s = 2; s < stage; ++s) {
-    const int64_t chunks = (a.n >> (kChunkBits + kStageBits * (s - 1))) + 1;
-    count += chunks;
-    if (s > 2) l += chunks * kListCap;
+  if (stage == 2) {
+    count = a.count + chunk;
+    return a.list1 + chunk * kListCap;
   }
-  count += chunk;
-  return l + chunk * kListCap;
+  count = a.count + (a.n >> (kChunkBits + kStageBits)) + 1;
+  return a.list2;
 }
 
 // Stage 1: one block per 256 bodies, thread t the binary node at base + t.
@@ -604,10 +603,7 @@ void launch_levels(int64_t n, Buffers &b, cudaStream_t s) {
 
 }  // namespace
 
-constexpr int64_t kChunkMax = 65536;
-
-void launch_upward(int64_t n, int L, int order, Buffers &b, cudaStream_t s) {
-  (void)L;
+void launch_upward(int64_t n, int order, Buffers &b, cudaStream_t s) {
   if (n > kChunkMax) {
     if (order >= 8) launch_levels<8>(n, b, s);
     else if (order >= 4) launch_levels<4>(n, b, s);

@@ -42,7 +42,8 @@ constexpr int kWalkBlocksPerSm = 16;
 // registers) against the compiler's own choice for FP64 (182 / 222 registers,
 // 11 / 9 warps per SM) took the FP64 walk at 2^20 from 15.5 to 12.3 ms
 // (quadrupole) and from 29.4 to 26.3 ms (octupole, despite 592 bytes of
-// spills; 12 blocks: 27.1 ms), the same bits.
+// spills; 12 blocks: 27.1 ms), the same bits.  Of the FP64 octupole walk, whose
+// block has 13,696 bytes of shared memory, 15 fit on an SM.
 template <typename T, int ORDER> constexpr int walk_min_blocks() { return kWalkBlocksPerSm; }
 constexpr int kCellQ = 64;
 constexpr int kBodyPerLane = 16;

@@ -40,7 +40,9 @@ extern "C" {
 #define BH_PREC_REFERENCE 2  /* per-target FP64 walk with the reference's MAC        */
 #define BH_PREC_DEHNEN 3     /* Dehnen's dual-tree method in FP64 (octree_default.f90
                                 :1095-1712, methods 20/21/22); the call synchronises
-                                its stream once and cannot be captured in a graph    */
+                                its stream at least once (its pair lists are sized
+                                from counts read back) and cannot be captured in a
+                                graph                                                */
 
 typedef struct bh_params {
     double theta;     /* opening angle, unsquared                                 */
@@ -72,7 +74,7 @@ typedef struct bh_params {
                          1 producer warps walk the tree and hand the batches on
                          through a shared-memory ring, consumer warps evaluate them
                          (the same results bit for bit; no reference counterpart;
-                         large FP64 walks stay on one warp per group)              */
+                         FP64 walks of many groups stay on one warp per group)     */
 } bh_params;
 
 /* Defaults: theta 0.5, G 1, eps 0, order 4, forces, depth 21, FP32, amp 1.2,
