@@ -36,8 +36,12 @@ struct bh_system {
   bh_params walk_p{};
   double *walk_out = nullptr;
   int walk_g0 = 0, walk_g1 = -1;  // its target groups (bh_system_walk_groups)
-  // captured build + walk of the current layout
+  // captured build + walk of the current layout, and what they work on: a replay
+  // that has to be completed (strict keys, stack growth) repeats its own work
   cudaGraphExec_t graph = nullptr;
+  bh_params graph_p{};
+  double *graph_out = nullptr;
+  const double *graph_in[4] = {nullptr, nullptr, nullptr, nullptr};
   // pinned staging of the layout's reduction items; the event marks the end
   // of the last layout upload, after which ss_host and items_pin may be reused
   bh::RedItem *items_pin = nullptr;
@@ -718,6 +722,8 @@ int bh_system_capture(bh_system *s, const bh_params *p, double *d_out) {
   BH_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   const bh_params saved = s->p;
   const int saved_order = s->order;
+  s->walk_g0 = 0;  // every group, whatever range was walked last
+  s->walk_g1 = -1;
   s->p = *p;
   s->order = p->order;
   cudaGraph_t g = nullptr;
@@ -737,8 +743,9 @@ int bh_system_capture(bh_system *s, const bh_params *p, double *d_out) {
     cudaGetLastError();
     return set_err(BH_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
   }
-  s->walk_p = *p;
-  s->walk_out = d_out;
+  s->graph_p = *p;
+  s->graph_out = d_out;
+  s->graph_in[0] = s->m; s->graph_in[1] = s->x; s->graph_in[2] = s->y; s->graph_in[3] = s->z;
   s->built = 0;  // nothing ran yet: the first replay builds
   return BH_OK;
 }
@@ -748,6 +755,12 @@ int bh_system_replay(bh_system *s, void *stream) {
   if (!s->graph) return set_err(BH_ERR_NOT_BUILT, "replay before capture");
   BH_CUDA(cudaSetDevice(s->device));
   BH_CUDA(cudaGraphLaunch(s->graph, (cudaStream_t)stream));
+  s->m = s->graph_in[0]; s->x = s->graph_in[1]; s->y = s->graph_in[2]; s->z = s->graph_in[3];
+  s->p = s->walk_p = s->graph_p;
+  s->order = s->graph_p.order;
+  s->walk_out = s->graph_out;
+  s->walk_g0 = 0;
+  s->walk_g1 = -1;
   s->built = 1;
   s->walked = 1;
   s->keys_checked = s->p.strict_keys ? 0 : 1;

@@ -158,7 +158,8 @@ class BHSystem:
     def capture(self, params: BHParams, out: torch.Tensor) -> None:
         """Records build + walk of the current batch (same input tensors,
         layout and parameters) into a CUDA graph held by the handle."""
-        self._graph_out = out
+        self._graph_out = out  # the graph reads and writes these
+        self._graph_inputs = self._inputs
         check(lib().bh_system_capture(self._h, C.byref(params), _dptr(out)))
 
     def replay(self) -> None:

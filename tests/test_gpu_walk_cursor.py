@@ -131,3 +131,27 @@ def test_replay_that_runs_out_of_stack(system):
     system.replay()
     system.sync()  # repeats the walk with a larger stack
     assert torch.equal(out, ref)
+
+
+def test_replay_repeats_its_own_walk(system):
+    """The walk that is repeated because a replay ran out of stack is the graph's:
+    its parameters, output, inputs and all groups, whatever was built and walked
+    between the capture and the replay."""
+    m, q = wide_deep_bodies()
+    args = [torch.from_numpy(a).cuda() for a in (m, *xyz(q))]
+    kw = dict(leaf_cap=1, amp=1.0 + 2.0 ** -23, strict_keys=0)
+    p, other = _params(theta=0.0, **kw), _params(theta=0.9, order=1, **kw)
+    ref = _plain(args, p)
+    out = torch.full_like(ref, float("nan"))
+    mine = torch.full_like(ref, 7.0)
+    system.build(*args, p)
+    system.walk(p, torch.empty_like(ref), groups=(0, 1))
+    system.capture(p, out)
+    system.build(args[0] * 2.0, *args[1:], other)
+    system.walk(other, mine, groups=(0, 1))
+    system.sync()
+    kept = mine.clone()
+    system.replay()
+    system.sync()
+    assert torch.equal(out, ref)
+    assert torch.equal(mine, kept)
