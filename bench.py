@@ -217,6 +217,38 @@ def launches_per_evaluation(n, nsys=1, L=21):
     return keys + sort + tree + upward + groups + walk
 
 
+def walk_kernel(n, p):
+    """The kernel that walks one system of n bodies with parameters p (the rule of
+    choose_walk in bh_walk.cu for a lone system)."""
+    if p.precision == 2:
+        return "reference_walk_kernel"
+    if p.precision == 3:
+        return "eval_kernel"
+    if not p.pipeline:
+        return "group_walk_kernel"
+    groups = math.ceil(n / p.group_size)
+    if p.precision == 1:
+        most = min(max(40 * math.sqrt(n), 800), {1: 2400, 4: 5000, 8: 2900}[p.order])
+        return "wide_walk_kernel" if groups <= most else "group_walk_kernel"
+    most = 1024 if p.order < 8 else (768 if p.group_size == 64 else 1400)
+    return "wide_walk_kernel" if groups <= most else "team_walk_kernel"
+
+
+def captured_traffic(kernel, n, p):
+    """DRAM bytes of one launch of that kernel from the committed capture, or None
+    when the capture is of another kernel or another workload."""
+    tf = os.path.join(ROOT, "profiles", "walk_dram_traffic.json")
+    if not os.path.exists(tf):
+        return None
+    with open(tf) as fh:
+        c = json.load(fh)
+    w = c["workload"]
+    same = c["kernel"] == kernel and w["n"] == n and all(
+        getattr(p, k) == w[k] for k in ("theta", "eps", "order", "precision", "group_size", "leaf_cap",
+                                        "group_span", "mac", "pipeline"))
+    return c["dram_bytes_read"] + c["dram_bytes_write"] if same else None
+
+
 def dist_max(x, dev, world):
     if world == 1:
         return x
@@ -482,17 +514,13 @@ def run_ours(args):
         exe_flops = float(st[0]) * FLOPS_PP + float(st[1]) * FLOPS_PC[args.order]
         t_w = statistics.mean(t_walk) * 1e-3
         achieved = alg_flops / t_w / 1e12
-        traffic = None
-        tf = os.path.join(ROOT, "profiles", "walk_dram_traffic.json")
-        if os.path.exists(tf):
-            with open(tf) as fh:
-                traffic = json.load(fh).get("bytes_per_launch_scaled")
+        kernel = walk_kernel(n, p)
         line["roofline"] = {
             "bound": "fp32",
-            "kernel": "team_walk_kernel" if p.pipeline and args.precision == 0 else "group_walk_kernel",
+            "kernel": kernel,
             "achieved": achieved,
             "peak": fp32_peak / 1e3, "unit": "TFLOP/s", "frac": achieved / (fp32_peak / 1e3),
-            "traffic": traffic,
+            "traffic": captured_traffic(kernel, n, p),
             "peak_source": "FP32 FMA throughput measured by bh_probe_fma_peak in this run, the larger "
                            "of scalar and paired (f32x2) FMA chains "
                            "(MEASURED_PEAKS.json has no FP32 figure; its HBM copy peak is not the bound)",
