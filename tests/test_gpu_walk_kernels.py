@@ -126,3 +126,30 @@ def test_many_small_systems_do_not_wait_for_producers(systems, n, order, precisi
             best[k] = min(best[k], a.elapsed_time(b) / 10)
     s.close()
     assert best[1] <= 1.5 * best[0], best
+
+
+@pytest.mark.parametrize("n,order,precision,group_size", [
+    (153600, 1, 1, 64), (153601, 1, 1, 64), (320000, 4, 1, 64), (320001, 4, 1, 64),
+    (185600, 8, 1, 64), (185601, 8, 1, 64), (12800, 8, 0, 32), (12801, 8, 0, 32),
+    (44800, 8, 0, 32), (44801, 8, 0, 32), (10240, 4, 0, 32), (10241, 4, 0, 32)])
+def test_both_sides_of_a_line_in_groups(n, order, precision, group_size):
+    _same(*_cloud(n, 3), order=order, precision=precision, group_size=group_size, theta=0.9, eps=0.0)
+
+
+@pytest.mark.parametrize("groups", [1, 319, 320, 321, 1024, 1025])
+def test_ranges_of_groups(groups):
+    """A range of a large system's groups goes to the kernel of that many groups."""
+    from hierarquicos_b200._lib import default_params
+    from hierarquicos_b200.system import BHSystem
+
+    m, q = _cloud(150000, 8)
+    s = BHSystem()
+    params = [default_params(order=4, theta=0.7, eps=0.01, pipeline=p) for p in (0, 1)]
+    s.build(m, q[:, 0], q[:, 1], q[:, 2], params[0])
+    s.sync()
+    outs = [torch.zeros(3 * len(m), dtype=torch.float64, device="cuda") for _ in params]
+    for p, out in zip(params, outs):
+        s.walk(p, out, groups=(700, 700 + groups))
+        s.sync()
+    s.close()
+    assert torch.equal(*outs) and 0 < int((outs[0] != 0).sum()) <= 3 * 64 * groups
